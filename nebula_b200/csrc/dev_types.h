@@ -51,6 +51,7 @@ struct Geometry {
     const int32_t* octree;
     const float4* tri;        // per triangle: (r0, mat_in), (e1, mat_out), (e2, 0)
     const float4* tri_face;   // per triangle: (e1 x e2, (mat_out << 16) | (mat_in & 0xFFFF))
+    const float4* tri_plane;  // per triangle: (n, n . r0), n the normal of length 1 / rounding margin (nm)
     float cx, cy, cz, hx, hy, hz;
     float max_extent;
     int n_tri;

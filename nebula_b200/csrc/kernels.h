@@ -156,8 +156,10 @@ cudaError_t launch_transport(const dev::Physics& P, const TransportArgs& a, int 
                              cudaStream_t s, int mode = kModePlain);
 int transport_max_blocks_per_sm(int block, int variant, int mode = kModePlain);
 // Per-triangle face records (normal e1 x e2 and packed materials) for
-// Geometry::tri_face; materials must fit in 16 bits.
-cudaError_t launch_triangle_faces(const float4* tri, float4* face, int n, cudaStream_t s);
+// Geometry::tri_face; materials must fit in 16 bits; and plane records for
+// Geometry::tri_plane, `scale` the largest coordinate of the domain.
+cudaError_t launch_triangle_faces(const float4* tri, float4* face, float4* plane, int n, float scale,
+                                  cudaStream_t s);
 // Surface map over [lo, lo + n * cell): each cell searches the candidate
 // list of its brick of `brick`^3 cells (brick_tris[brick_start[b] ..
 // brick_start[b + 1]), bricks x-fastest over nbx x nby x ...) for the nearest

@@ -94,7 +94,7 @@ struct nbx_ctx {
     // geometry
     DevBuf<int32_t> octree;
     DevBuf<float4> tris;
-    DevBuf<float4> tri_faces;
+    DevBuf<float4> tri_faces, tri_planes;
     // energy-deposit records (kDepositWords floats each) and the device cursor
     DevBuf<float> dep;
     DevBuf<unsigned long long> dep_cursor;
@@ -612,12 +612,17 @@ int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* o) {
         ctx->tris.alloc(t.size());
         to_device(ctx, ctx->tris.p, t.data(), sizeof(float4) * t.size(), "triangles");
         ctx->tri_faces.alloc(std::max<uint64_t>(o->n_triangles, 1));
-        ck(nbx::launch_triangle_faces(ctx->tris.p, ctx->tri_faces.p, int(o->n_triangles), ctx->stream), "faces");
+        ctx->tri_planes.alloc(std::max<uint64_t>(o->n_triangles, 1));
+        float scale = 0;   // largest coordinate of the domain
+        for (int i = 0; i < 3; ++i) scale = std::max(scale, std::fabs(o->center[i]) + o->halfsize[i]);
+        ck(nbx::launch_triangle_faces(ctx->tris.p, ctx->tri_faces.p, ctx->tri_planes.p, int(o->n_triangles), scale,
+                                      ctx->stream), "faces");
         ck(cudaStreamSynchronize(ctx->stream), "faces");
         auto& g = ctx->phys.geo;
         g.octree = ctx->octree.p;
         g.tri = ctx->tris.p;
         g.tri_face = ctx->tri_faces.p;
+        g.tri_plane = ctx->tri_planes.p;
         g.cx = o->center[0];
         g.cy = o->center[1];
         g.cz = o->center[2];

@@ -783,12 +783,33 @@ __global__ void pixel_yields_kernel(const uint32_t* se, const uint32_t* bse, con
 // Face records: e1 x e2 computed with the transport's arithmetic (the same
 // expression propagate and boundary would evaluate) and both materials packed
 // as 16-bit halves.
-__global__ void triangle_faces_kernel(const float4* tri, float4* face, int n) {
+// Plane records for the early rejection (plane_misses): the unit normal and
+// the plane's offset, from double precision, both divided by the margin that
+// covers the rounding of the exact test.  With u = 2^-24, the shape factor
+// k = |e1||e2| / |e1 x e2| and positions at most `scale` from the origin
+// (3.5 scale apart), intersect_ray's numerator e2 . (s x e1) is off by at most
+// 12 u |s||e1||e2|, i.e. 2.5e-6 k scale of plane distance, its determinant by
+// 8 u |e1||e2|, which moves a plane at distance r by 8 u k r <= 1.7e-6 k scale;
+// the rejection's own two dot products add less than 1e-6 scale.  A margin
+// above 1 nm (slivers) gets a zero record, which never rejects.
+__global__ void triangle_faces_kernel(const float4* tri, float4* face, float4* plane, int n, float scale) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 b = tri[3 * i + 1], c = tri[3 * i + 2];
         const dev::V3 nrm = dev::cross(dev::V3{b.x, b.y, b.z}, dev::V3{c.x, c.y, c.z});
         const uint32_t mi = uint32_t(__float_as_int(tri[3 * i].w)), mo = uint32_t(__float_as_int(b.w));
         face[i] = make_float4(nrm.x, nrm.y, nrm.z, __uint_as_float((mo << 16) | (mi & 0xFFFFu)));
+        const double bx = b.x, by = b.y, bz = b.z, cx = c.x, cy = c.y, cz = c.z;
+        const double nx = by * cz - bz * cy, ny = bz * cx - bx * cz, nz = bx * cy - by * cx;
+        const double len = sqrt(nx * nx + ny * ny + nz * nz);
+        const double edges = sqrt((bx * bx + by * by + bz * bz) * (cx * cx + cy * cy + cz * cz));
+        float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const double margin = (5e-6 * edges / len + 1e-6) * scale;
+        if (len > 0.0 && edges < 1e30 && margin < 1.0) {
+            const float4 a = tri[3 * i];
+            const double k = 1.0 / (len * margin);
+            p = make_float4(float(k * nx), float(k * ny), float(k * nz), float(k * (nx * a.x + ny * a.y + nz * a.z)));
+        }
+        plane[i] = p;
     }
 }
 
@@ -990,9 +1011,10 @@ __global__ void features_kernel(const dev::SurfaceMap S, const ElectronRecord* e
 }
 }  // namespace
 
-cudaError_t launch_triangle_faces(const float4* tri, float4* face, int n, cudaStream_t s) {
+cudaError_t launch_triangle_faces(const float4* tri, float4* face, float4* plane, int n, float scale,
+                                  cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    triangle_faces_kernel<<<grid_for(uint64_t(n), 256), 256, 0, s>>>(tri, face, n);
+    triangle_faces_kernel<<<grid_for(uint64_t(n), 256), 256, 0, s>>>(tri, face, plane, n, scale);
     return cudaGetLastError();
 }
 
