@@ -182,7 +182,7 @@ typedef struct {
     uint64_t record_capacity;  /* detected records held on the device; 0 = auto */
     int32_t block_size;        /* threads per block of the transport kernel; 0 = 256 */
     int32_t blocks_per_sm;     /* transport variant: 2, 3 or 4 resident 256-thread blocks per SM, or 7
-                                  128-thread blocks (block_size capped at 128); 0 = 4 (64 registers) */
+                                  128-thread blocks (block_size capped at 128); 0 = 3 (80 registers) */
     int32_t inelastic_model;   /* NBX_INELASTIC_KIEFT (0, default) or NBX_INELASTIC_FULL_PENN */
     int32_t record_deposits;   /* keep energy-deposit records (plain mode; cpu_energydep.cpp) */
     uint64_t deposit_capacity; /* deposit records held on the device; 0 = 2^27 (3.2 GB) */
@@ -327,8 +327,9 @@ typedef struct {
     int32_t blocks_per_sm;   /* transport variant: 2, 3 or 4 resident 256-thread blocks per SM, or 7
                                 resident 128-thread blocks */
     int32_t block_size;      /* threads per block (multiple of 32; at most 128 for variant 7) */
-    int32_t stack_depth;     /* parked ancestors per thread (1..64, default 16): a secondary born deeper
-                                in its cascade goes to the next generation's queue */
+    int32_t stack_depth;     /* parked electrons per thread (1..64, default 16), shared by the 32 threads of
+                                a warp: a secondary born with its warp's stack full goes to the next
+                                generation's queue (sample mode: each thread its own stack) */
     int32_t chunk;           /* generation launches queued between two host reads (1..64, default 8) */
     uint64_t queue_capacity; /* out: entries of each overflow queue in the last run */
     double sample_ms;        /* out (nbx_autotune): the sample's device time with these settings */

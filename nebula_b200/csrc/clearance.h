@@ -1,0 +1,25 @@
+// Clearance map of a geometry (see clearance.cu): built on the device when the
+// geometry is set, used by the transport to skip the octree walk of steps that
+// cannot meet a triangle.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "dev_types.h"
+
+namespace nbx {
+
+struct ClearanceMap {
+    dev::Clearance map{};   // what the kernels take; map.top == nullptr: no map
+    int* top = nullptr;     // device buffers behind it
+    float4* rec = nullptr;
+};
+
+// Builds the map of `n_tri` triangles (three float4 each, device memory) over
+// the octree's root box.  False (and nothing allocated) when the memory for it
+// is not there or a launch failed: the transport then walks every step.
+bool build_clearance(const float4* tri, int n_tri, const float center[3], const float half[3], int sms, cudaStream_t s,
+                     ClearanceMap* out);
+void free_clearance(ClearanceMap* m);
+
+}  // namespace nbx

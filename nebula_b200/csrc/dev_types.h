@@ -46,12 +46,26 @@ struct Material {
     Table2D el_icdf, in_icdf, ion;
     Table3D q, ion3;
 };
+// Clearance map (clearance.cu): a coarse grid (nx x ny x ..., x fastest) over
+// the octree's root box whose cells are empty (kClearNear: no triangle within
+// `reach`, kClearFar: none within `far_reach`) or index a brick of 4 x 4 x 4
+// slab records (n, c), one per fine cell of edge h.
+constexpr int kClearNear = -1, kClearFar = -2;
+struct Clearance {
+    const int* top;           // nullptr: no map
+    const float4* rec;
+    float lox, loy, loz;
+    float h, inv_h;
+    int nx, ny;
+    float reach, far_reach;
+};
 // Triangles as three float4: (r0, mat_in bits), (e1, mat_out bits), (e2, 0).
 struct Geometry {
     const int32_t* octree;
     const float4* tri;        // per triangle: (r0, mat_in), (e1, mat_out), (e2, 0)
     const float4* tri_face;   // per triangle: (e1 x e2, (mat_out << 16) | (mat_in & 0xFFFF))
     const float4* tri_plane;  // per triangle: (n, n . r0), n the normal of length 1 / rounding margin (nm)
+    Clearance clear;
     float cx, cy, cz, hx, hy, hz;
     float max_extent;
     int n_tri;

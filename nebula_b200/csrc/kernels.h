@@ -118,10 +118,10 @@ struct TransportArgs {
     float* dep;
     unsigned long long* dep_cursor;   // records handed out (chunks of kDepositChunk)
     unsigned long long dep_capacity;  // records the buffer holds
-    // parked-ancestor stacks, 3 * stack_depth float4 per launched thread
-    // (nullptr: a local-memory array of kLocalStack entries)
-    float4* stack_mem;
-    int stack_depth;            // 1 .. kMaxStack: parked ancestors per thread in stack_mem
+    // parked electrons: transport_stack_bytes of the launch (nullptr: local
+    // memory, kLocalStack entries per thread; not in sample mode)
+    uint32_t* stack_mem;
+    int stack_depth;            // 1 .. kMaxStack: parked electrons per thread in stack_mem
     // per-pixel exit spectra (nullptr: off): pix_spec[pixel * pix_bins + bin]
     // counts (weights in learned mode) of detections, pixel = pixel_of_tag[tag]
     float* pix_spec;
@@ -139,19 +139,22 @@ constexpr uint32_t kDepositChunk = 32;
 constexpr uint32_t kDepositEmpty = 0xFFFFFFFFu;
 
 // kModeLearned: weighted transport, the network evaluated on the tensor
-// cores for every newborn (warp-synchronous); kModeWeighted: weighted
-// transport whose birth decisions come from the network's importance table
-// or the fixed rule (no warp-synchronous step).
+// cores for every newborn; kModeWeighted: weighted transport whose birth
+// decisions come from the network's importance table or the fixed rule.
 enum : int { kModePlain = 0, kModeSample = 1, kModeLearned = 2, kModeDeposit = 3, kModeWeighted = 4 };
 
-// Per-thread stack of parked ancestors (depth-first cascades): the depth of
-// the local-memory array used without a stack buffer, and the largest depth
-// a stack buffer may be given.
+// Stack of parked electrons (depth-first cascades): entries per thread of the
+// local-memory array used without a stack buffer, and the most a stack buffer
+// may be given.  A warp's threads share theirs; kDeepSlack more entries per
+// warp (a multiple of 32) hold what its lanes and its ring own at most when
+// the stack is full (32 + 40).
 constexpr int kLocalStack = 16;
 constexpr int kMaxStack = 64;
+constexpr int kDeepSlack = 96;
+uint64_t transport_stack_bytes(int grid, int block, int depth, int mode);
 
-// variant: resident blocks per SM the kernel was compiled for (2, 3 or 4);
-// mode: kModePlain, kModeSample or kModeLearned.
+// variant: resident blocks per SM the kernel was compiled for (2, 3, 4 or 7);
+// mode: kModePlain .. kModeWeighted.
 cudaError_t launch_transport(const dev::Physics& P, const TransportArgs& a, int grid, int block, int variant,
                              cudaStream_t s, int mode = kModePlain);
 int transport_max_blocks_per_sm(int block, int variant, int mode = kModePlain);

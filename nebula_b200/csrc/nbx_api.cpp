@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 
+#include "clearance.h"
 #include "kernels.h"
 #include "material.h"
 #include "mlp.cuh"
@@ -95,6 +96,7 @@ struct nbx_ctx {
     DevBuf<int32_t> octree;
     DevBuf<float4> tris;
     DevBuf<float4> tri_faces, tri_planes;
+    nbx::ClearanceMap clearance;
     // energy-deposit records (kDepositWords floats each) and the device cursor
     DevBuf<float> dep;
     DevBuf<unsigned long long> dep_cursor;
@@ -155,7 +157,7 @@ struct nbx_ctx {
     DevBuf<uint32_t> sample_count;
     uint64_t sample_cap = 0;
     DevBuf<float> se_w, bse_w;
-    DevBuf<float4> stack_mem;     // transport parked-ancestor stacks (grow-only)
+    DevBuf<uint32_t> stack_mem;   // transport stacks of parked electrons (grow-only)
     DevBuf<uint32_t> range_cursor; // per-SM pop cursors of the primary generation (grow-only)
     DevBuf<uint32_t> yield_map;   // nbx_pixel_yields work buffers (grow-only)
     uint64_t pixel_map_len = 0;    // tags covered by a map from nbx_set_pixel_map
@@ -170,7 +172,7 @@ struct nbx_ctx {
     uint64_t pushed = 0, generations = 0;
     double last_run_ms = 0, last_kernel_ms = 0;
     int block = 256, bpsm = 0, variant = 3;
-    int stack_depth = 16;   // parked ancestors per thread before a secondary goes to the next generation
+    int stack_depth = 16;   // parked electrons per thread before a secondary goes to the next generation
     int chunk = 8;          // generation launches queued between two 4-byte host reads
     uint64_t queue_capacity = 0;   // overflow-queue entries of the last run
     // device address of the allocation-free transport's scratch array,
@@ -179,6 +181,7 @@ struct nbx_ctx {
 
     ~nbx_ctx() {
         for (auto* t : tables) delete t;
+        nbx::free_clearance(&clearance);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (staged_ev) cudaEventDestroy(staged_ev);
@@ -550,9 +553,10 @@ int nbx_create(nbx_ctx** out, const nbx_config* cfg) {
         if (ctx->block % 32 != 0 || ctx->block > 256) throw ApiError(NBX_ERR_ARG, "block_size must be a multiple of 32, <= 256");
         // Kernel variant = resident blocks per SM it was register-limited for:
         // 2, 3 or 4 blocks of 256 threads, or 7 blocks of 128 (72 registers;
-        // block size capped at 128); default 4 (64 registers: the
-        // autotuner's choice on most workloads).
-        ctx->variant = ((c.blocks_per_sm >= 2 && c.blocks_per_sm <= 4) || c.blocks_per_sm == 7) ? c.blocks_per_sm : 4;
+        // block size capped at 128).  Default 3 (80 registers): 64 spill in
+        // the walk (grating 9.42e9 against 9.86e9 events/s, contact holes
+        // 3.48e9 against 3.86e9, rough slab equal), 128 leave too few warps.
+        ctx->variant = ((c.blocks_per_sm >= 2 && c.blocks_per_sm <= 4) || c.blocks_per_sm == 7) ? c.blocks_per_sm : 3;
         if (ctx->variant == 7 && ctx->block > 128) ctx->block = 128;
         ctx->bpsm = nbx::transport_max_blocks_per_sm(ctx->block, ctx->variant);
         if (c.record_deposits) {
@@ -623,6 +627,13 @@ int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* o) {
         g.tri = ctx->tris.p;
         g.tri_face = ctx->tri_faces.p;
         g.tri_plane = ctx->tri_planes.p;
+        // without memory for the map the transport walks every step
+        nbx::free_clearance(&ctx->clearance);
+        if (nbx::build_clearance(ctx->tris.p, int(o->n_triangles), o->center, o->halfsize, ctx->sms, ctx->stream,
+                                 &ctx->clearance))
+            g.clear = ctx->clearance.map;
+        else
+            g.clear = nbx::dev::Clearance{};
         g.cx = o->center[0];
         g.cy = o->center[1];
         g.cz = o->center[2];
@@ -959,8 +970,8 @@ int nbx_run(nbx_ctx* ctx) {
         }
         const int bpsm = nbx::transport_max_blocks_per_sm(ctx->block, ctx->variant, mode);
         const int grid = ctx->sms * bpsm;
-        // parked-ancestor stacks of the launched threads (grow-only)
-        ctx->stack_mem.ensure(uint64_t(grid) * uint64_t(ctx->block) * 3 * uint64_t(ctx->stack_depth));
+        // stacks of parked electrons of the launched warps (grow-only)
+        ctx->stack_mem.ensure(nbx::transport_stack_bytes(grid, ctx->block, ctx->stack_depth, mode) / sizeof(uint32_t));
         a.stack_mem = ctx->stack_mem.p;
         a.stack_depth = ctx->stack_depth;
         // The primaries are popped from per-SM ranges (neighbouring queue

@@ -3,22 +3,19 @@
 // The transport kernel replaces the reference's event-sorted SIMT driver
 // (drivers/gpu/gpu_driver.inl:312-567: init + CUB radix sort + intersect /
 // elastic / inelastic launched over the whole slot capacity every
-// iteration).  Here each thread keeps one electron in registers and runs
-// init -> event passes back to back until the electron terminates or is
-// detected, then refills from a device queue with a warp-aggregated atomic.
-// Cascades run depth-first, child first: when an event creates a secondary,
-// the parent is parked on a small per-thread stack and the secondary is
-// simulated at once, so a primary's whole cascade normally stays in one
-// thread and never touches global memory.  Only a cascade deeper than the
-// stack hands secondaries to the next generation's queue (warp-aggregated
-// push).  Detections are tallied per primary tag on the device; detected
-// records are optional.
+// iteration).  Here every warp keeps a pool of electrons in registers and
+// shared memory and advances them step by step until all have terminated or
+// been detected, refilling from a device queue.  Cascades run depth-first,
+// child first: when an event creates a secondary, the parent is parked on the
+// warp's stack and the secondary is simulated at once, so a primary's whole
+// cascade normally stays in one warp.  Only a secondary born with the stack
+// full goes to the next generation's queue.  Detections are tallied per
+// primary tag on the device; detected records are optional.
 #include <cooperative_groups.h>
 #include <cooperative_groups/reduce.h>
 
 #include <algorithm>
 #include <mutex>
-#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -57,12 +54,6 @@ __device__ __forceinline__ void store_electron(const Queue& q, uint32_t i, const
     q.c[i] = make_uint4(e.tag, uint32_t(e.uid), uint32_t(e.uid >> 32), uint32_t(e.last_tri));
 }
 
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // Learned mode: statistical weights are powers of two, 2^wexp, so every
 // roulette survivor's weight 1 / q is exact and fits in a few bits of the
 // parked material word; wexp stays within [kMinWeightExp, kMaxWeightExp].
@@ -72,16 +63,6 @@ constexpr int kMinWeightExp = -4;   // at least 1/16 (a chain of splits)
 // exponent in the queue's last-triangle word (a secondary has no last
 // triangle): kWeightTag | uint8(wexp); no real triangle index has these bits.
 constexpr uint32_t kWeightTag = 0xFFFFFE00u;
-
-// Words per thread of the transport kernel's dynamic shared memory: the leaf
-// cache, then the event counters.  Counter slots 0-3 are indexed by the event
-// type (dev::kEvNone .. dev::kEvBoundary; slot 0 is never read).
-constexpr int kLeafCacheWords = 13;
-constexpr int kSlotSteps = 4, kSlotSecondaries = 5, kSlotDetectedSE = 6, kSlotDetectedBSE = 7, kSlotTerminated = 8,
-              kSlotPopped = 9;
-constexpr int kCounterSlots = 10;
-static_assert(dev::kEvNone == 0 && dev::kEvInelastic == 1 && dev::kEvElastic == 2 && dev::kEvBoundary == 3,
-              "event types index counter slots 0-3");
 
 struct LearnedSmem {
     mlp::Weights w;
@@ -115,76 +96,6 @@ __device__ __noinline__ float birth_logit(unsigned m, bool cand, const dev::Surf
     const float mine = __shfl_sync(0xffffffffu, logit, rank);
     __syncwarp();
     return mine;
-}
-
-// Per-electron state of the sample mode, parked alongside the electron.
-struct Extra {
-    int rec;          // sample record slot, -1 none
-    uint32_t flags;   // bit 0: sub-cascade produced a detected SE
-    uint32_t c0;      // the thread's step count when the record was taken
-};
-
-// Parked ancestors of a thread's cascade, in global memory laid out per
-// thread (stack_depth entries of three float4: (pos, E), (dir, material),
-// (uid, step, last triangle)).  A local-memory array interleaves threads word
-// by word, so lanes parked at different depths scatter each of an entry's 13
-// words into its own sector; here an entry is 48 contiguous bytes (two
-// sectors, three 16-byte accesses).  The tag is not stored: every electron of
-// a thread's cascade carries its primary's tag.  With kW (learned mode) the
-// material word also carries the weight exponent in its upper 16 bits (the
-// material index fits the lower 16).  base == nullptr: use the local array
-// instead (callers without a stack buffer).
-struct ParkedStack {
-    float4* base;
-    template <bool kW>
-    __device__ __forceinline__ void put(int i, const dev::Electron& e, dev::Electron* local, int wexp) const {
-        const int mw = kW ? int((uint32_t(e.mat) & 0xFFFFu) | (uint32_t(wexp) << 16)) : e.mat;
-        if (base) {
-            float4* p = base + 3 * i;
-            p[0] = make_float4(e.px, e.py, e.pz, e.E);
-            p[1] = make_float4(e.dx, e.dy, e.dz, __int_as_float(mw));
-            p[2] = make_float4(__uint_as_float(uint32_t(e.uid)), __uint_as_float(uint32_t(e.uid >> 32)),
-                               __uint_as_float(e.step), __int_as_float(e.last_tri));
-        } else {
-            local[i] = e;
-            local[i].mat = mw;
-        }
-    }
-    template <bool kW>
-    __device__ __forceinline__ void get(int i, dev::Electron& e, const dev::Electron* local, int& wexp) const {
-        int mw;
-        if (base) {
-            const float4* p = base + 3 * i;
-            const float4 a = p[0], b = p[1], c = p[2];
-            e.px = a.x;
-            e.py = a.y;
-            e.pz = a.z;
-            e.E = a.w;
-            e.dx = b.x;
-            e.dy = b.y;
-            e.dz = b.z;
-            mw = __float_as_int(b.w);
-            e.uid = uint64_t(__float_as_uint(c.x)) | (uint64_t(__float_as_uint(c.y)) << 32);
-            e.step = __float_as_uint(c.z);
-            e.last_tri = __float_as_int(c.w);
-        } else {
-            e = local[i];
-            mw = e.mat;
-        }
-        if constexpr (kW) {
-            e.mat = int(int16_t(mw & 0xFFFF));
-            wexp = mw >> 16;
-        } else {
-            e.mat = mw;
-        }
-    }
-};
-
-__device__ __forceinline__ uint32_t mix32(uint64_t x) {
-    x ^= x >> 33;
-    x *= 0xFF51AFD7ED558CCDull;
-    x ^= x >> 33;
-    return uint32_t(x);
 }
 
 // Philox block of a secondary's step 0 that decides its roulette at birth
@@ -241,39 +152,153 @@ __device__ __forceinline__ float table_importance(const TransportArgs& a, const 
     return __ldg(a.imp_table + ((size_t(m) * a.imp_ne + ie) * a.imp_nd + id) * a.imp_nc + ic);
 }
 
+// ---------------------------------------------------------------------------
+// The transport kernel: every warp keeps a pool of electrons and its lanes
+// take them step by step, so that the lanes of one instruction do the same
+// work.
+//
+// Measured before (one thread per cascade, all lanes in one divergent loop):
+// 9.7 of 32 lanes active per instruction and 78 % of the issue slots busy on
+// the grating, and a small scan took as long as its longest cascade run by one
+// thread.  Two things caused the divergence: the octree walk (a few lanes of a
+// warp in different cells and list lengths at any time) and the cascades'
+// bookkeeping.  Now
+//
+// * a step whose free path the clearance map answers goes straight on to its
+//   scattering event; one that needs the walk (about one in eight) goes to the
+//   warp's ring in shared memory and its lane takes other work.  When
+//   kWalkBatch of them wait, or too few lanes have other work, the warp walks
+//   them together, one electron per lane; those that met a triangle cross (or
+//   leave) there, the others come back for their scattering event.
+// * parked electrons (the parents of running secondaries) lie on one stack per
+//   warp, its top kTop entries in shared memory, the rest in the warp's part
+//   of stack_mem, so any lane that falls idle takes the next one: a cascade
+//   spreads over the warp.  Child first, as before, which keeps the stack
+//   short.
+//
+// An electron's draws depend only on its own stream (uid, step), so the order
+// in which lanes take electrons changes no result.
+//
+// B200, against one thread per cascade without the map (both with the plane
+// rejection): half the benchmark's grating frame 129.0 -> 98.2 ms, rough slab
+// 46.4 -> 22.8 ms, contact holes 51.8 -> 41.0 ms, a 1,024-primary tile 3.66 ->
+// 0.85 ms; 30 of 32 lanes hold an electron, 25 of them finish an event per
+// pass through the loop.
+// ---------------------------------------------------------------------------
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kStateWords = 13;                // an electron
+constexpr int kWalkWords = kStateWords + 4;    // + path, code, two uniforms' bits
+constexpr int kRing = 40;                      // ring slots
+constexpr int kTop = 32;                       // stack entries in shared memory
+constexpr int kWarpWords = kRing * kWalkWords + kTop * kStateWords;
+// Waiting electrons that start a walk.  The ring holds up to 32 that came back
+// and the ones that queue up meanwhile: 24 keeps the walk's lanes mostly full
+// and leaves room.
+constexpr int kWalkBatch = 24;
+// Ring codes: the scattering event that waits (1 inelastic, 2 elastic, as in
+// the walk's input; 0: none, the step starts in vacuum), an electron whose next
+// step starts, one that ended.
+constexpr int kCodeFresh = 3, kCodeEnded = 4;
+
+// Counters of a warp: lane k keeps counter k (kCnt*) of its warp, so a tally is
+// one predicated add on a warp-uniform count.
+static_assert(kNumCounters <= 32, "one lane per counter");
+
+template <bool kW>
+__device__ __forceinline__ void put_state(uint32_t* p, int stride, const dev::Electron& e, int wexp) {
+    p[0] = __float_as_uint(e.px);
+    p[stride] = __float_as_uint(e.py);
+    p[2 * stride] = __float_as_uint(e.pz);
+    p[3 * stride] = __float_as_uint(e.E);
+    p[4 * stride] = __float_as_uint(e.dx);
+    p[5 * stride] = __float_as_uint(e.dy);
+    p[6 * stride] = __float_as_uint(e.dz);
+    // learned mode: the weight exponent in the upper half (materials fit 16 bits)
+    p[7 * stride] = kW ? ((uint32_t(e.mat) & 0xFFFFu) | (uint32_t(wexp) << 16)) : uint32_t(e.mat);
+    p[8 * stride] = uint32_t(e.last_tri);
+    p[9 * stride] = e.tag;
+    p[10 * stride] = uint32_t(e.uid);
+    p[11 * stride] = uint32_t(e.uid >> 32);
+    p[12 * stride] = e.step;
+}
+template <bool kW>
+__device__ __forceinline__ void get_state(const uint32_t* p, int stride, dev::Electron& e, int& wexp) {
+    e.px = __uint_as_float(p[0]);
+    e.py = __uint_as_float(p[stride]);
+    e.pz = __uint_as_float(p[2 * stride]);
+    e.E = __uint_as_float(p[3 * stride]);
+    e.dx = __uint_as_float(p[4 * stride]);
+    e.dy = __uint_as_float(p[5 * stride]);
+    e.dz = __uint_as_float(p[6 * stride]);
+    const uint32_t m = p[7 * stride];
+    e.mat = kW ? int(int16_t(m & 0xFFFFu)) : int(m);
+    if constexpr (kW) wexp = int(m) >> 16;
+    e.last_tri = int(p[8 * stride]);
+    e.tag = p[9 * stride];
+    e.uid = uint64_t(p[10 * stride]) | (uint64_t(p[11 * stride]) << 32);
+    e.step = p[12 * stride];
+}
+
+// Tallies of one detected electron of weight 2^wexp.
+template <bool kW>
+__device__ __forceinline__ void tally_detected(const TransportArgs& a, const dev::Electron& e, int wexp) {
+    const bool is_se = e.E < 50;
+    [[maybe_unused]] const float wt = kW ? ldexpf(1.0f, wexp) : 1.0f;
+    if (e.tag < a.n_tags) {
+        atomicAdd(is_se ? a.se_count + e.tag : a.bse_count + e.tag, 1u);
+        if constexpr (kW) atomicAdd(is_se ? a.se_w + e.tag : a.bse_w + e.tag, wt);
+    }
+    if (a.hist) {
+        int bin = dev::floor_to_int(e.E * a.inv_bin_width);
+        bin = bin < 0 ? 0 : (bin >= a.n_bins ? a.n_bins - 1 : bin);
+        atomicAdd(a.hist + bin, 1ull);
+    }
+    if (a.pix_spec && e.tag < a.n_map) {
+        // per-pixel exit spectrum; energies past the last bin are not binned
+        const uint32_t px = a.pixel_of_tag[e.tag];
+        const int bin = dev::floor_to_int(e.E * a.pix_inv_width);
+        if (px < a.n_pixels && bin >= 0 && bin < a.pix_bins) atomicAdd(a.pix_spec + size_t(px) * a.pix_bins + bin, wt);
+    }
+    if (a.rec) {
+        const uint32_t slot = atomicAdd(a.rec_count, 1u);
+        if (slot < a.rec_capacity) {
+            a.rec[2 * size_t(slot)] = make_float4(e.px, e.py, e.pz, e.dx);
+            a.rec[2 * size_t(slot) + 1] = make_float4(e.dy, e.dz, e.E, __uint_as_float(e.tag));
+        } else {
+            atomicAdd(a.counters + kCntRecordsDropped, 1ull);
+        }
+    }
+}
+
 // MinBlocks: resident blocks per SM the register allocation must allow --
 // 256-thread blocks for 2 (128 registers), 3 (80) and 4 (64); 128-thread
 // blocks for 7 (72 registers, 28 warps); the host picks the variant.
-// Mode: kModePlain (analogue transport), kModeSample (plain transport that
-// also records one (features, label, cost) training sample for about one in
-// sixteen newborn secondaries), kModeLearned (plain transport of weighted
-// electrons: every newborn secondary is scored at birth by the network,
-// batched per warp on the tensor cores, and plays Russian roulette or splits
-// on that importance; a warp stays in the loop until all its lanes are done,
-// so the tensor-core call always has the whole warp), or kModeDeposit (plain
-// transport that also appends an energy-deposit record per energy-changing
-// scattering event).
+// Mode: kModePlain (analogue transport), kModeLearned (weighted electrons:
+// every newborn secondary is scored at birth by the network, batched per warp
+// on the tensor cores, and plays Russian roulette or splits on that
+// importance), kModeWeighted (the same decided by the importance table or the
+// fixed rule), or kModeDeposit (plain transport that also appends an
+// energy-deposit record per energy-changing scattering event).
 template <int MinBlocks, int Mode, bool Penn>
 __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transport_kernel(const dev::Physics P, const TransportArgs a) {
-    // Dynamic shared memory sized by the launch (transport_smem_bytes), per
-    // thread and strided by the block size: the leaf cache (13 words), then
-    // the thread's event counters (kCounterSlots words), so a 128-thread
-    // block does not hold a 256-thread allocation and the rest of the SM's
-    // L1 stays with the cascade stacks.  The counters live there rather than
-    // in registers, which the octree walk needs: a shared-memory atomic add
-    // per event costs one instruction, as a register increment does.
-    extern __shared__ float leaf_cache[];
-    const dev::LeafCache cache{leaf_cache + threadIdx.x, int(blockDim.x)};
-    cache.f(0) = 0.0f;   // location 0: empty
-    cache.f(1) = 0.0f;
-    uint32_t* const cnt = reinterpret_cast<uint32_t*>(leaf_cache + kLeafCacheWords * blockDim.x) + threadIdx.x;
-    const int cs = int(blockDim.x);
-#pragma unroll
-    for (int k = 0; k < kCounterSlots; ++k) cnt[k * cs] = 0u;
-    auto bump = [&](int slot) { atomicAdd(cnt + slot * cs, 1u); };
-    constexpr bool kExtra = (Mode == kModeSample);
-    constexpr bool kNet = (Mode == kModeLearned);                   // tensor-core inference at birth
+    constexpr bool kNet = (Mode == kModeLearned);                          // tensor-core inference at birth
     constexpr bool kW = (Mode == kModeLearned || Mode == kModeWeighted);   // weighted electrons
+    extern __shared__ uint32_t pool_words[];
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t* const ring = pool_words + (threadIdx.x >> 5) * kWarpWords;
+    uint32_t* const top = ring + kRing * kWalkWords;
+    // The stack's deep part: 32 * stack_depth parked electrons plus room for
+    // what the ring and the lanes hold (a warp never owns more than the
+    // stack's limit plus those), word by word; without a stack buffer, in the
+    // lanes' local memory, entry i in lane i % 32.
+    const int limit = 32 * (a.stack_mem ? a.stack_depth : kLocalStack);
+    const int deep_cap = limit + kDeepSlack;
+    uint32_t* const deep = a.stack_mem ? a.stack_mem + (size_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) *
+                                                           (size_t(kStateWords) * deep_cap)
+                                       : nullptr;
+    uint32_t local_deep[kLocalStack + kDeepSlack / 32][kStateWords];
+
     bool use_net = false, use_rule = false;
     int rule_k = 0;
     if constexpr (kW) {
@@ -292,32 +317,81 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
         }
     }
     const uint32_t n_in = min(*a.n_in, a.in_capacity);
-    dev::Electron e;
-    // Child-first depth-first cascade: when an event creates a secondary the
-    // parent is parked here and the secondary is simulated at once, so the
-    // stack only ever holds the current electron's ancestors.
-    dev::Electron stack[kLocalStack];
-    const ParkedStack ps{a.stack_mem ? a.stack_mem + (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 3 * a.stack_depth
-                                     : nullptr};
-    const int depth = a.stack_mem ? a.stack_depth : kLocalStack;
-    Extra ex{-1, 0u, 0u};
-    Extra exs[kExtra ? kMaxStack : 1];
-    int wexp = 0;   // learned mode: the current electron's weight is 2^wexp
-    int sp = 0;
-    bool alive = false, drained = false;
-    uint32_t probe = 0;   // ranges this thread has found used up (range_cursor)
-    uint32_t carry_hit = 0;
-    // Per-thread tallies in 32 bits (a thread would need 2^32 steps in one
-    // launch to wrap): the frequent ones in the shared-memory slots above,
-    // the weighted, sample and deposit modes' own in registers; rare ones
-    // (dropped records, queue overflow) go straight to the global counters.
-    uint32_t c_inf = 0, c_kill = 0, c_split = 0, c_smp = 0, c_dep = 0, c_dep_drop = 0;
-    // Deposit mode: this thread's current chunk [dep_pos, dep_end) of the
+
+    // This lane's electron, and what it waits for.
+    dev::Electron e{};
+    int wexp = 0;   // learned mode: its weight is 2^wexp
+    // The warp's pool (all warp-uniform): ring slots [head, head + n_back) are
+    // back from the walk, [head + n_back, head + n_back + n_wait) wait for it;
+    // top_n entries of the stack in shared memory, deep_n below them.
+    int head = 0, n_back = 0, n_wait = 0, top_n = 0, deep_n = 0;
+    bool have = false, drained = false;
+    // Primaries: this SM's range of the queue first, then the following ones
+    // (`probe` ranges found used up).
+    uint32_t probe = 0, taken = 0;
+    int warps_log2 = 0;   // warps that share a cursor
+    {
+        const uint32_t w = gridDim.x * (blockDim.x >> 5) / (a.range_cursor ? a.n_ranges : 1u);
+        while ((1u << warps_log2) < w) ++warps_log2;
+    }
+    unsigned long long mine = 0;   // this lane's counter (kCnt* = lane)
+    auto count = [&](int which, unsigned mask) {
+        if (lane == which) mine += __popc(mask);
+    };
+    // Deposit mode: this lane's current chunk [dep_pos, dep_end) of the
     // record buffer, taken kDepositChunk records at a time with one atomic.
-    unsigned long long dep_pos = 0, dep_end = 0;
-    bool dep_full = false;
-    // Hand an electron to the next generation's queue (warp-aggregated push
-    // over the lanes that push together).
+    [[maybe_unused]] unsigned long long dep_pos = 0, dep_end = 0;
+    [[maybe_unused]] bool dep_full = false;
+
+    auto slot_at = [&](int i) {
+        i += head;
+        i -= i >= kRing ? kRing : 0;
+        return ring + (i >= kRing ? i - kRing : i);
+    };
+    // Moves stack entries [0, n) of the shared part to or from the deep
+    // entries [at, at + n); entry at + i goes through lane (at + i) % 32, which
+    // owns it when the deep part is local memory.
+    auto move_deep = [&](int at, int n, bool out) {
+        const int i = (lane - at) & 31;
+        if (i < n) {
+            uint32_t* const t = top + i;
+            if (deep) {
+                uint32_t* const d = deep + at + i;
+                if (out) {
+#pragma unroll
+                    for (int k = 0; k < kStateWords; ++k) d[size_t(k) * deep_cap] = t[k * kTop];
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kStateWords; ++k) t[k * kTop] = d[size_t(k) * deep_cap];
+                }
+            } else {
+                uint32_t* const d = local_deep[(at + i) >> 5];
+                if (out) {
+#pragma unroll
+                    for (int k = 0; k < kStateWords; ++k) d[k] = t[k * kTop];
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kStateWords; ++k) t[k * kTop] = d[k];
+                }
+            }
+        }
+        __syncwarp();
+    };
+    // Pushes the electrons of the lanes in `mask` on the warp's stack (the
+    // caller has made sure that they fit).
+    auto push = [&](unsigned mask, const dev::Electron& x, int x_wexp) {
+        const int n = __popc(mask);
+        if (top_n + n > kTop) {
+            move_deep(deep_n, top_n, true);
+            deep_n += top_n;
+            top_n = 0;
+        }
+        if ((mask >> lane) & 1u) put_state<kW>(top + top_n + __popc(mask & below), kTop, x, x_wexp);
+        top_n += n;
+        __syncwarp();
+    };
+    // Hands a newborn secondary to the next generation's queue
+    // (warp-aggregated over the lanes that call together).
     auto push_next = [&](const dev::Electron& x, int x_wexp) {
         cg::coalesced_group g = cg::coalesced_threads();
         uint32_t base = 0;
@@ -333,16 +407,418 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
             atomicAdd(a.counters + kCntOverflow, 1ull);
         }
     };
-    for (;;) {
-        if (!alive && !drained) {
-            if (sp > 0) {
-                ps.get<kW>(--sp, e, stack, wexp);
-                if constexpr (kExtra) {
-                    ex = exs[sp];
-                    ex.flags |= carry_hit;
-                    carry_hit = 0;
+    // The octree walk of the waiting electrons, one per lane; crossings and
+    // exits happen here, a waiting scattering event is left to the main loop.
+    auto walk = [&] {
+        const int n = min(n_wait, 32);
+        const bool on = lane < n;
+        bool stepped = false, crossed = false, init_end = false, ended = false, se = false, bse = false;
+        if (on) {
+            uint32_t* const q = slot_at(n_back + lane);
+            dev::Electron w;
+            int w_wexp = 0;
+            get_state<kW>(q, kRing, w, w_wexp);
+            const float dist = __uint_as_float(q[13 * kRing]);
+            const int type = int(q[14 * kRing]);
+            const dev::V3 nd = dev::normalised(dev::V3{w.dx, w.dy, w.dz});
+            int hit;
+            const float t = dev::propagate(P.geo, dev::V3{w.px, w.py, w.pz}, nd, dist, w.last_tri, w.mat, &hit);
+            if (hit >= 0 || type == 0) {
+                stepped = true;
+                crossed = hit >= 0;
+                const int st = dev::cross(P, w, nd, t, hit, q[15 * kRing]);
+                if (st == dev::kDetected) {
+                    se = w.E < 50;
+                    bse = !se;
+                    tally_detected<kW>(a, w, w_wexp);
+                } else {
+                    // the next init pass would only end the electron: that step too
+                    init_end = st == dev::kAlive && dev::ends_at_init(P, w);
+                    ended = init_end || st == dev::kTerminated;
                 }
-                alive = true;
+                const bool over = ended || se || bse;
+                if (!over) put_state<kW>(q, kRing, w, w_wexp);
+                q[14 * kRing] = over ? kCodeEnded : kCodeFresh;
+            }
+        }
+        count(kCntSteps, __ballot_sync(kFull, stepped));
+        count(kCntBoundary, __ballot_sync(kFull, crossed));
+        count(kCntDetectedSE, __ballot_sync(kFull, se));
+        count(kCntDetectedBSE, __ballot_sync(kFull, bse));
+        count(kCntTerminated, __ballot_sync(kFull, ended));
+        const unsigned extra = __ballot_sync(kFull, init_end);
+        if (extra) count(kCntSteps, extra);
+        n_back += n;
+        n_wait -= n;
+        __syncwarp();
+    };
+
+    for (;;) {
+        // Every electron a lane holds here is about to start a step.
+        if (n_wait > 0 && n_back == 0) {
+            const bool other_work = !drained || top_n + deep_n > 0;
+            if (n_wait >= kWalkBatch || (!other_work && n_wait >= __popc(__ballot_sync(kFull, have)))) walk();
+        }
+        // -- idle lanes take work: back from the walk, then parked, then a
+        // primary
+        int code = kCodeFresh;
+        float dist = 0.0f;
+        uint32_t rz = 0, rw = 0;
+        const unsigned idle = __ballot_sync(kFull, !have);
+        if (idle) {
+            const int want = __popc(idle), rank = have ? 64 : __popc(idle & below);
+            const int n1 = min(want, n_back);
+            if (n1 > 0) {
+                if (rank < n1) {
+                    const uint32_t* const q = slot_at(rank);
+                    code = int(q[14 * kRing]);
+                    if (code != kCodeEnded) {
+                        get_state<kW>(q, kRing, e, wexp);
+                        dist = __uint_as_float(q[13 * kRing]);
+                        rz = q[15 * kRing];
+                        rw = q[16 * kRing];
+                        have = true;
+                    }
+                }
+                head += n1;
+                head -= head >= kRing ? kRing : 0;
+                n_back -= n1;
+                __syncwarp();
+            }
+            if (want > n1) {
+                if (top_n == 0 && deep_n > 0) {
+                    const int n = min(deep_n, kTop);
+                    deep_n -= n;
+                    move_deep(deep_n, n, false);
+                    top_n = n;
+                }
+                const int n2 = min(want - n1, top_n);
+                if (n2 > 0) {
+                    const int r = rank - n1;
+                    if (r >= 0 && r < n2) {
+                        get_state<kW>(top + (top_n - 1 - r), kTop, e, wexp);
+                        have = true;
+                    }
+                    top_n -= n2;
+                    __syncwarp();
+                }
+                const int open = want - n1 - n2;
+                if (open > 0 && deep_n == 0 && !drained) {
+                    // Primaries: all open lanes' worth while the range holds
+                    // plenty, a warp's share of what is left toward its end
+                    // (so a small batch spreads over the warps).
+                    uint32_t lo = 0, len = n_in;
+                    uint32_t* cursor = a.head;
+                    if (a.range_cursor) {
+                        uint32_t smid;
+                        asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+                        uint32_t v = smid % a.n_ranges + probe;
+                        if (v >= a.n_ranges) v -= a.n_ranges;
+                        lo = uint32_t(uint64_t(n_in) * v / a.n_ranges);
+                        len = uint32_t(uint64_t(n_in) * (v + 1) / a.n_ranges) - lo;
+                        cursor = a.range_cursor + v;
+                    }
+                    const uint32_t ask = min(uint32_t(open), max(1u, (len - min(taken, len)) >> warps_log2));
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(cursor, ask);
+                    base = __shfl_sync(kFull, base, 0);
+                    const uint32_t got = base < len ? min(ask, len - base) : 0u;
+                    taken = base + got;
+                    if (got < ask) {
+                        taken = 0;
+                        ++probe;
+                        drained = !a.range_cursor || probe >= a.n_ranges;
+                    }
+                    const int r = rank - n1 - n2;
+                    bool ended = false;
+                    if (r >= 0 && uint32_t(r) < got) {
+                        load_electron(a.in, lo + base + uint32_t(r), e);
+                        if constexpr (kW) {
+                            wexp = 0;
+                            if ((uint32_t(e.last_tri) & 0xFFFFFF00u) == kWeightTag) {
+                                wexp = int(int8_t(uint32_t(e.last_tri) & 0xFFu));
+                                e.last_tri = -1;
+                            }
+                        }
+                        ended = dev::ends_at_init(P, e);
+                        have = !ended;
+                    }
+                    if (lane == kCntPopped) mine += got;
+                    const unsigned m = __ballot_sync(kFull, ended);
+                    count(kCntSteps, m);
+                    count(kCntTerminated, m);
+                }
+            }
+        }
+        const unsigned busy = __ballot_sync(kFull, have);
+        if (!busy) {
+            if (drained && n_back + n_wait + top_n + deep_n == 0) break;
+            continue;
+        }
+
+        // -- a step's first half: free paths, and whether they need the walk
+        const dev::V3 nd = dev::normalised(dev::V3{e.dx, e.dy, e.dz});
+        bool need_walk = false;
+        if (have && code == kCodeFresh) {
+            const uint4 r = dev::draw(P.seed, e, 0);
+            rz = r.z;
+            rw = r.w;
+            dev::free_path(P, e, r, &code, &dist);
+            need_walk = !(code != 0 && dev::step_is_clear(P.geo.clear, dev::V3{e.px, e.py, e.pz}, nd, dist));
+        }
+        const unsigned walkers = __ballot_sync(kFull, need_walk);
+        if (walkers) {
+            const int n = __popc(walkers), room = kRing - n_back - n_wait, r = __popc(walkers & below);
+            if (need_walk && r < room) {
+                uint32_t* const q = slot_at(n_back + n_wait + r);
+                put_state<kW>(q, kRing, e, wexp);
+                q[13 * kRing] = __float_as_uint(dist);
+                q[14 * kRing] = uint32_t(code);
+                q[15 * kRing] = rz;
+                q[16 * kRing] = rw;
+            }
+            n_wait += min(n, room);
+            // no room: back to the stack, to start this step again later
+            if (n > room) push(__ballot_sync(kFull, need_walk && r >= room), e, wexp);
+            if (need_walk) have = false;
+            __syncwarp();
+        }
+
+        // -- second half: the scattering event
+        bool has_se = false;
+        dev::Electron se;
+        const bool event = have;
+        const bool inelastic = event && code == dev::kEvInelastic;
+        [[maybe_unused]] const float E_before = e.E;
+        if (event) dev::scatter<Penn>(P, e, nd, dist, code, rz, rw, &se, &has_se);
+        {
+            const unsigned m = __ballot_sync(kFull, event), mi = __ballot_sync(kFull, inelastic);
+            count(kCntSteps, m);
+            count(kCntInelastic, mi);
+            count(kCntElastic, m & ~mi);
+            count(kCntSecondaries, __ballot_sync(kFull, has_se));
+        }
+        if constexpr (Mode == kModeDeposit) {
+            // energydeposit_cpu_driver::simulate_to_end (drivers/cpu/
+            // energydeposit_cpu_driver.h:74-96): scattering events only, and
+            // only when the energy changed; position after the event.
+            bool kept = false, lost = false;
+            if (event && e.E != E_before) {
+                if (dep_pos == dep_end && !dep_full) {
+                    const unsigned long long base = atomicAdd(a.dep_cursor, (unsigned long long)kDepositChunk);
+                    if (base + kDepositChunk <= a.dep_capacity) {
+                        dep_pos = base;
+                        dep_end = base + kDepositChunk;
+                    } else {
+                        dep_full = true;
+                    }
+                }
+                kept = dep_pos < dep_end;
+                lost = !kept;
+                if (kept) {
+                    float* r = a.dep + dep_pos * kDepositWords;
+                    r[0] = e.px;
+                    r[1] = e.py;
+                    r[2] = e.pz;
+                    r[3] = E_before;
+                    r[4] = E_before - e.E;
+                    r[5] = __uint_as_float(e.tag);
+                    ++dep_pos;
+                }
+            }
+            count(kCntDeposits, __ballot_sync(kFull, kept));
+            count(kCntDepositsDropped, __ballot_sync(kFull, lost));
+        }
+
+        // -- the secondary.  Init passes that would only end an electron
+        // (outside the domain, or an energy outside the material's range) are
+        // tallied now: about a quarter of the secondaries start below the
+        // barrier.
+        const bool se_dead = has_se && dev::ends_at_init(P, se);
+        bool se_runs = has_se && !se_dead;
+        // Learned mode: birth decision for every newborn secondary of the warp
+        // (k > 0 roulette at survival 2^-k, -1 split, 0 keep).  The network
+        // scores the warp's candidates together: they are packed into the
+        // first rows of the warp's feature tile and one (up to 16 candidates)
+        // or two m-tiles go through the tensor cores.
+        int se_wexp = wexp;
+        bool split = false;
+        if constexpr (kW) {
+            int bk = 0;
+            bool drop = false;
+            if (use_rule) {
+                // roulette up to the rule's weight 2^rule_k: a newborn that
+                // already carries it (its ancestor survived the rule) is kept
+                if (se_runs && wexp < rule_k && se.E < a.birth_max_energy &&
+                    dev::surface_distance(a.smap, se.px, se.py, se.pz) >= a.birth_min_distance)
+                    bk = rule_k - wexp;
+            } else if (use_net) {
+                const unsigned m = __ballot_sync(kFull, se_runs);
+                if constexpr (kNet) {
+                    if (m) {
+                        const float logit =
+                            birth_logit(m, se_runs, a.smap, se.px, se.py, se.pz, se.dx, se.dy, se.dz, se.E, se.mat);
+                        count(kCntInferences, 1u);
+                        if (se_runs) bk = birth_decision(a, mlp::sigmoid(logit), wexp, se.E, se.mat);
+                    }
+                } else {
+                    count(kCntInferences, m);
+                    if (se_runs) bk = birth_decision(a, table_importance(a, se), wexp, se.E, se.mat);
+                }
+            }
+            if (bk > 0) {
+                // Russian roulette: survive with probability 2^-bk at weight
+                // 2^(wexp + bk); the draw is the secondary's own birth block
+                if (wexp + bk > kMaxWeightExp) bk = kMaxWeightExp - wexp;
+                if (bk > 0 && !(ldexpf(dev::u01(dev::draw(P.seed, se, kBirthBlock).x), bk) < 1.0f)) drop = true;
+            } else if (bk < 0 && wexp <= kMinWeightExp) {
+                bk = 0;   // the lineage is already split as far as it may be
+            }
+            count(kCntRouletteKilled, __ballot_sync(kFull, drop));
+            se_runs = se_runs && !drop;
+            // the newborn's weight exponent: roulette survivors gain bk, both
+            // halves of a split lose one
+            se_wexp = wexp + (bk < 0 ? -1 : bk);
+            split = se_runs && bk < 0;
+        }
+        const bool e_dead = event && dev::ends_at_init(P, e);
+        {
+            const unsigned m = __ballot_sync(kFull, se_dead), me = __ballot_sync(kFull, e_dead);
+            if (lane == kCntSteps || lane == kCntTerminated) mine += __popc(m) + __popc(me);
+        }
+        if constexpr (kW) {
+            // split: the twin takes its own random streams
+            const unsigned m = __ballot_sync(kFull, split);
+            if (m) {
+                count(kCntSplit, m);
+                dev::Electron twin = se;
+                if (split) twin.uid = dev::secondary_uid(se.uid ^ 0x5DEECE66Dull, 0u);
+                if (top_n + deep_n + __popc(m) <= limit) push(m, twin, se_wexp);
+                else if (split) push_next(twin, se_wexp);
+            }
+        }
+        // Child first: the parent is parked and the secondary runs on in this
+        // lane; with the stack full the secondary goes to the next generation.
+        const unsigned parents = __ballot_sync(kFull, se_runs && !e_dead);
+        if (parents) {
+            if (top_n + deep_n + __popc(parents) <= limit) {
+                push(parents, e, wexp);
+            } else if (se_runs && !e_dead) {
+                push_next(se, se_wexp);
+                se_runs = false;
+            }
+        }
+        if (se_runs) {
+            e = se;
+            wexp = se_wexp;
+        } else if (e_dead) {
+            have = false;
+        }
+    }
+    if constexpr (Mode == kModeDeposit) {
+        // mark the unused tail of this thread's last chunk
+        for (; dep_pos < dep_end; ++dep_pos) a.dep[dep_pos * kDepositWords + 5] = __uint_as_float(kDepositEmpty);
+    }
+    if (lane == kCntDetected) mine = 0;
+    const unsigned long long n_se = __shfl_sync(kFull, mine, kCntDetectedSE), n_bse = __shfl_sync(kFull, mine, kCntDetectedBSE);
+    if (lane == kCntDetected) mine = n_se + n_bse;
+    if (lane < kNumCounters && mine) atomicAdd(a.counters + lane, mine);
+}
+
+// ---------------------------------------------------------------------------
+// Sample mode (training data): plain transport that also records one
+// (features, label, cost) sample for about one in sixteen newborn secondaries.
+// A thread runs a primary's whole cascade, child first, on its own stack, so
+// a sample's sub-cascade is a contiguous run of the thread's steps: its cost is
+// a difference of the thread's step count, and its label is passed up as the
+// children finish.  (The transport kernel's pool spreads a cascade over a
+// warp, where neither holds.)
+// ---------------------------------------------------------------------------
+
+// Words per thread of the sample kernel's dynamic shared memory: the leaf
+// cache, then the event counters.  Counter slots 0-3 are indexed by the event
+// type (dev::kEvNone .. dev::kEvBoundary; slot 0 is never read).
+constexpr int kLeafCacheWords = 13;
+constexpr int kSlotSteps = 4, kSlotSecondaries = 5, kSlotDetectedSE = 6, kSlotDetectedBSE = 7, kSlotTerminated = 8,
+              kSlotPopped = 9;
+constexpr int kCounterSlots = 10;
+static_assert(dev::kEvNone == 0 && dev::kEvInelastic == 1 && dev::kEvElastic == 2 && dev::kEvBoundary == 3,
+              "event types index counter slots 0-3");
+
+// Per-electron state of the sample mode, parked alongside the electron.
+struct Extra {
+    int rec;          // sample record slot, -1 none
+    uint32_t flags;   // bit 0: sub-cascade produced a detected SE
+    uint32_t c0;      // the thread's step count when the record was taken
+};
+
+// Parked ancestors of a thread's cascade, in global memory laid out per
+// thread (stack_depth entries of three float4: (pos, E), (dir, material),
+// (uid, step, last triangle)): an entry is 48 contiguous bytes.  The tag is
+// not stored: every electron of a thread's cascade carries its primary's tag.
+__device__ __forceinline__ void park(float4* p, const dev::Electron& e) {
+    p[0] = make_float4(e.px, e.py, e.pz, e.E);
+    p[1] = make_float4(e.dx, e.dy, e.dz, __int_as_float(e.mat));
+    p[2] = make_float4(__uint_as_float(uint32_t(e.uid)), __uint_as_float(uint32_t(e.uid >> 32)),
+                       __uint_as_float(e.step), __int_as_float(e.last_tri));
+}
+__device__ __forceinline__ void unpark(const float4* p, dev::Electron& e) {
+    const float4 a = p[0], b = p[1], c = p[2];
+    e.px = a.x;
+    e.py = a.y;
+    e.pz = a.z;
+    e.E = a.w;
+    e.dx = b.x;
+    e.dy = b.y;
+    e.dz = b.z;
+    e.mat = __float_as_int(b.w);
+    e.uid = uint64_t(__float_as_uint(c.x)) | (uint64_t(__float_as_uint(c.y)) << 32);
+    e.step = __float_as_uint(c.z);
+    e.last_tri = __float_as_int(c.w);
+}
+
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ uint32_t mix32(uint64_t x) {
+    x ^= x >> 33;
+    x *= 0xFF51AFD7ED558CCDull;
+    x ^= x >> 33;
+    return uint32_t(x);
+}
+
+// Variants as transport_kernel's.  Primaries are popped warp-aggregated from
+// this SM's range of the queue, as there.
+template <int MinBlocks, bool Penn>
+__global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) sample_kernel(const dev::Physics P, const TransportArgs a) {
+    extern __shared__ float leaf_cache[];
+    const dev::LeafCache cache{leaf_cache + threadIdx.x, int(blockDim.x)};
+    cache.f(0) = 0.0f;   // location 0: empty
+    cache.f(1) = 0.0f;
+    uint32_t* const cnt = reinterpret_cast<uint32_t*>(leaf_cache + kLeafCacheWords * blockDim.x) + threadIdx.x;
+    const int cs = int(blockDim.x);
+#pragma unroll
+    for (int k = 0; k < kCounterSlots; ++k) cnt[k * cs] = 0u;
+    auto bump = [&](int slot) { atomicAdd(cnt + slot * cs, 1u); };
+    const uint32_t n_in = min(*a.n_in, a.in_capacity);
+    dev::Electron e;
+    float4* const stack = reinterpret_cast<float4*>(a.stack_mem) + (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 3 * a.stack_depth;
+    Extra ex{-1, 0u, 0u};
+    Extra exs[kMaxStack];
+    int sp = 0;
+    uint32_t probe = 0;   // ranges this thread has found used up (range_cursor)
+    uint32_t carry_hit = 0, c_smp = 0;
+    bool alive = false;
+    for (;;) {
+        if (!alive) {
+            if (sp > 0) {
+                unpark(stack + 3 * --sp, e);
+                ex = exs[sp];
+                ex.flags |= carry_hit;
+                carry_hit = 0;
             } else {
                 uint32_t idx = 0;
                 bool got = false;
@@ -377,175 +853,64 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
                     idx = base + g.thread_rank();
                     got = idx < n_in;
                 }
-                if (!got) {
-                    drained = true;
-                } else {
-                    load_electron(a.in, idx, e);
-                    if constexpr (kW) {
-                        wexp = 0;
-                        if ((uint32_t(e.last_tri) & 0xFFFFFF00u) == kWeightTag) {
-                            wexp = int(int8_t(uint32_t(e.last_tri) & 0xFFu));
-                            e.last_tri = -1;
-                        }
-                    }
-                    if constexpr (kExtra) {
-                        ex.rec = -1;
-                        ex.flags = 0;
-                        carry_hit = 0;
-                    }
-                    bump(kSlotPopped);
-                    alive = true;
-                }
+                if (!got) break;
+                load_electron(a.in, idx, e);
+                ex.rec = -1;
+                ex.flags = 0;
+                carry_hit = 0;
+                bump(kSlotPopped);
             }
+            alive = true;
         }
-        if constexpr (kNet) {
-            // the whole warp stays in the loop until all its lanes are done
-            // (the tensor-core call at birth needs every lane)
-            if (__all_sync(0xffffffffu, !alive)) break;
-        } else {
-            if (!alive) break;
-        }
-        if constexpr (Mode == kModeSample) {
-            // one in sixteen electrons is recorded at its birth (step 0) in a
-            // material: features now; label and sub-cascade cost when it ends
-            if (ex.rec < 0 && e.step == 0 && e.mat >= 0 && (mix32(e.uid) & 15u) == 0) {
-                const uint32_t slot = atomicAdd(a.sample_count, 1u);
-                if (slot < a.sample_capacity) {
-                    float f[6];
-                    const dev::V3 d = dev::normalised(dev::V3{e.dx, e.dy, e.dz});
-                    dev::electron_features(a.smap, e.px, e.py, e.pz, d.x, d.y, d.z, logf(e.E), e.mat, f);
+        // one in sixteen electrons is recorded at its birth (step 0) in a
+        // material: features now; label and sub-cascade cost when it ends
+        if (ex.rec < 0 && e.step == 0 && e.mat >= 0 && (mix32(e.uid) & 15u) == 0) {
+            const uint32_t slot = atomicAdd(a.sample_count, 1u);
+            if (slot < a.sample_capacity) {
+                float f[6];
+                const dev::V3 d = dev::normalised(dev::V3{e.dx, e.dy, e.dz});
+                dev::electron_features(a.smap, e.px, e.py, e.pz, d.x, d.y, d.z, logf(e.E), e.mat, f);
 #pragma unroll
-                    for (int k = 0; k < 6; ++k) a.sample_feat[size_t(slot) * 6 + k] = f[k];
-                    ex.rec = int(slot);
-                    ex.c0 = cnt[kSlotSteps * cs];
-                    ++c_smp;
-                }
+                for (int k = 0; k < 6; ++k) a.sample_feat[size_t(slot) * 6 + k] = f[k];
+                ex.rec = int(slot);
+                ex.c0 = cnt[kSlotSteps * cs];
+                ++c_smp;
             }
         }
         int ev = dev::kEvNone;
         bool has_se = false;
         dev::Electron se;
-        int st = dev::kAlive;
-        [[maybe_unused]] const float E_before = e.E;
-        if (!kNet || alive) {
-            st = dev::step<Penn>(P, e, &ev, &se, &has_se, cache);
-            bump(kSlotSteps);
-        }
-        // Learned mode: birth decision for every newborn secondary of the warp
-        // (k > 0 roulette at survival 2^-k, -1 split, 0 keep; drop = lost the
-        // roulette).  The network scores the warp's candidates together: they
-        // are packed into the first rows of the warp's feature tile and one
-        // (up to 16 candidates) or two m-tiles go through the tensor cores.
-        int bk = 0;
-        bool drop = false;
-        if constexpr (kW) {
-            const bool cand = has_se && !dev::ends_at_init(P, se);
-            if (use_rule) {
-                // roulette up to the rule's weight 2^rule_k: a newborn that
-                // already carries it (its ancestor survived the rule) is kept
-                if (cand && wexp < rule_k && se.E < a.birth_max_energy &&
-                    dev::surface_distance(a.smap, se.px, se.py, se.pz) >= a.birth_min_distance)
-                    bk = rule_k - wexp;
-            } else if (use_net) {
-                if constexpr (kNet) {
-                    const unsigned m = __ballot_sync(0xffffffffu, cand);
-                    if (m) {
-                        const float logit =
-                            birth_logit(m, cand, a.smap, se.px, se.py, se.pz, se.dx, se.dy, se.dz, se.E, se.mat);
-                        if ((threadIdx.x & 31) == 0) ++c_inf;
-                        if (cand) bk = birth_decision(a, mlp::sigmoid(logit), wexp, se.E, se.mat);
-                    }
-                } else if (cand) {
-                    ++c_inf;
-                    bk = birth_decision(a, table_importance(a, se), wexp, se.E, se.mat);
-                }
-            }
-            if (bk > 0) {
-                // Russian roulette: survive with probability 2^-bk at weight
-                // 2^(wexp + bk); the draw is the secondary's own birth block
-                if (wexp + bk > kMaxWeightExp) bk = kMaxWeightExp - wexp;
-                if (bk > 0 && !(ldexpf(dev::u01(dev::draw(P.seed, se, kBirthBlock).x), bk) < 1.0f)) drop = true;
-            } else if (bk < 0 && wexp <= kMinWeightExp) {
-                bk = 0;   // the lineage is already split as far as it may be
-            }
-            if constexpr (kNet) {
-                if (!alive) continue;
-            }
-        }
-        if constexpr (Mode == kModeDeposit) {
-            // energydeposit_cpu_driver::simulate_to_end (drivers/cpu/
-            // energydeposit_cpu_driver.h:74-96): scattering events only, and
-            // only when the energy changed; position after the event.
-            if ((ev == dev::kEvElastic || ev == dev::kEvInelastic) && e.E != E_before) {
-                if (dep_pos == dep_end && !dep_full) {
-                    const unsigned long long base = atomicAdd(a.dep_cursor, (unsigned long long)kDepositChunk);
-                    if (base + kDepositChunk <= a.dep_capacity) {
-                        dep_pos = base;
-                        dep_end = base + kDepositChunk;
-                    } else {
-                        dep_full = true;
-                    }
-                }
-                if (dep_pos < dep_end) {
-                    float* r = a.dep + dep_pos * kDepositWords;
-                    r[0] = e.px;
-                    r[1] = e.py;
-                    r[2] = e.pz;
-                    r[3] = E_before;
-                    r[4] = E_before - e.E;
-                    r[5] = __uint_as_float(e.tag);
-                    ++dep_pos;
-                    ++c_dep;
-                } else {
-                    ++c_dep_drop;
-                }
-            }
-        }
+        int st = dev::step<Penn, true>(P, e, &ev, &se, &has_se, cache);
+        bump(kSlotSteps);
         bump(ev);   // slots 1-3 count the event types; slot 0 (no event) is not read
         if (has_se) {
             // an inelastic step never ends its electron: st == kAlive here
             bump(kSlotSecondaries);
-            if (drop) {
-                ++c_kill;   // the secondary's sub-cascade is not simulated
-            } else if (dev::ends_at_init(P, se)) {
-                // The secondary's first step would only terminate it (about a
-                // quarter of them start below the barrier): tally that step
-                // here instead of parking the parent for it.
+            if (dev::ends_at_init(P, se)) {
+                // The secondary's first step would only terminate it: tally
+                // that step here instead of parking the parent for it.
                 bump(kSlotSteps);
                 bump(kSlotTerminated);
+            } else if (sp < a.stack_depth) {
+                park(stack + 3 * sp, e);
+                exs[sp] = ex;
+                ++sp;
+                e = se;
+                ex.rec = -1;
+                ex.flags = 0;
+                continue;
             } else {
-                // the newborn's weight exponent: roulette survivors gain bk,
-                // both halves of a split lose one
-                const int se_wexp = wexp + (bk < 0 ? -1 : bk);
-                if (bk < 0) {
-                    // split: the twin takes its own random streams
-                    dev::Electron twin = se;
-                    twin.uid = dev::secondary_uid(se.uid ^ 0x5DEECE66Dull, 0u);
-                    ++c_split;
-                    if (sp + 1 < depth) {
-                        ps.put<kW>(sp, e, stack, wexp);
-                        ps.put<kW>(sp + 1, twin, stack, se_wexp);
-                        sp += 2;
-                        e = se;
-                        wexp = se_wexp;
-                        continue;
-                    }
-                    push_next(twin, se_wexp);
-                }
-                if (sp < depth) {
-                    ps.put<kW>(sp, e, stack, wexp);
-                    if constexpr (kExtra) exs[sp] = ex;
-                    ++sp;
-                    e = se;
-                    wexp = se_wexp;
-                    if constexpr (kExtra) {
-                        ex.rec = -1;
-                        ex.flags = 0;
-                    }
-                    continue;
-                }
-                // Deep cascade: hand the secondary to the next generation.
-                push_next(se, se_wexp);
+                // Deep cascade: hand the secondary to the next generation
+                // (warp-aggregated push over the lanes that push together).
+                cg::coalesced_group g = cg::coalesced_threads();
+                uint32_t base = 0;
+                if (g.thread_rank() == 0) base = atomicAdd(a.out_tail, g.size());
+                base = g.shfl(base, 0);
+                const uint32_t slot = base + g.thread_rank();
+                if (slot < a.out_capacity)
+                    store_electron(a.out, slot, se);
+                else
+                    atomicAdd(a.counters + kCntOverflow, 1ull);
             }
         }
         if (st == dev::kAlive) {
@@ -560,51 +925,19 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
         if (st == dev::kTerminated) {
             bump(kSlotTerminated);
         } else {
-            // detected
-            const bool is_se = e.E < 50;
-            hit = is_se ? 1u : 0u;
-            bump(is_se ? kSlotDetectedSE : kSlotDetectedBSE);
-            [[maybe_unused]] const float wt = kW ? ldexpf(1.0f, wexp) : 1.0f;
-            if (e.tag < a.n_tags) {
-                atomicAdd(is_se ? a.se_count + e.tag : a.bse_count + e.tag, 1u);
-                if constexpr (kW) atomicAdd(is_se ? a.se_w + e.tag : a.bse_w + e.tag, wt);
-            }
-            if (a.hist) {
-                int bin = dev::floor_to_int(e.E * a.inv_bin_width);
-                bin = bin < 0 ? 0 : (bin >= a.n_bins ? a.n_bins - 1 : bin);
-                atomicAdd(a.hist + bin, 1ull);
-            }
-            if (a.pix_spec && e.tag < a.n_map) {
-                // per-pixel exit spectrum; energies past the last bin are not binned
-                const uint32_t px = a.pixel_of_tag[e.tag];
-                const int bin = dev::floor_to_int(e.E * a.pix_inv_width);
-                if (px < a.n_pixels && bin >= 0 && bin < a.pix_bins) atomicAdd(a.pix_spec + size_t(px) * a.pix_bins + bin, wt);
-            }
-            if (a.rec) {
-                const uint32_t slot = atomicAdd(a.rec_count, 1u);
-                if (slot < a.rec_capacity) {
-                    a.rec[2 * size_t(slot)] = make_float4(e.px, e.py, e.pz, e.dx);
-                    a.rec[2 * size_t(slot) + 1] = make_float4(e.dy, e.dz, e.E, __uint_as_float(e.tag));
-                } else {
-                    atomicAdd(a.counters + kCntRecordsDropped, 1ull);
-                }
-            }
+            hit = e.E < 50 ? 1u : 0u;
+            bump(hit ? kSlotDetectedSE : kSlotDetectedBSE);
+            tally_detected<false>(a, e, 0);
         }
-        if constexpr (Mode == kModeSample) {
-            const uint32_t sub = (ex.flags | hit) & 1u;
-            if (ex.rec >= 0) {
-                a.sample_label[ex.rec] = float(sub);
-                if (a.sample_cost) a.sample_cost[ex.rec] = float(cnt[kSlotSteps * cs] - ex.c0);
-            }
-            carry_hit = sub;
+        const uint32_t sub = (ex.flags | hit) & 1u;
+        if (ex.rec >= 0) {
+            a.sample_label[ex.rec] = float(sub);
+            if (a.sample_cost) a.sample_cost[ex.rec] = float(cnt[kSlotSteps * cs] - ex.c0);
         }
-    }
-    if constexpr (Mode == kModeDeposit) {
-        // mark the unused tail of this thread's last chunk
-        for (; dep_pos < dep_end; ++dep_pos) a.dep[dep_pos * kDepositWords + 5] = __uint_as_float(kDepositEmpty);
+        carry_hit = sub;
     }
     // Counters: one atomic per warp per counter.
-    unsigned long long v[kNumCounters];
+    unsigned long long v[kNumCounters] = {};
     v[kCntSteps] = cnt[kSlotSteps * cs];
     v[kCntElastic] = cnt[dev::kEvElastic * cs];
     v[kCntInelastic] = cnt[dev::kEvInelastic * cs];
@@ -614,15 +947,8 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
     v[kCntDetectedSE] = cnt[kSlotDetectedSE * cs];
     v[kCntDetectedBSE] = cnt[kSlotDetectedBSE * cs];
     v[kCntTerminated] = cnt[kSlotTerminated * cs];
-    v[kCntRecordsDropped] = 0;
-    v[kCntOverflow] = 0;
     v[kCntPopped] = cnt[kSlotPopped * cs];
-    v[kCntInferences] = c_inf;
-    v[kCntRouletteKilled] = c_kill;
-    v[kCntSplit] = c_split;
     v[kCntSamples] = c_smp;
-    v[kCntDeposits] = c_dep;
-    v[kCntDepositsDropped] = c_dep_drop;
     __syncwarp();
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -739,7 +1065,7 @@ __global__ void step_query_kernel(const dev::Physics P, ElectronRecord* el, uint
         dev::Electron se{};
         int ev;
         bool hs;
-        status[i] = P.penn ? dev::step<true>(P, e, &ev, &se, &hs) : dev::step<false>(P, e, &ev, &se, &hs);
+        status[i] = P.penn ? dev::step<true, false>(P, e, &ev, &se, &hs) : dev::step<false, false>(P, e, &ev, &se, &hs);
         event[i] = ev;
         has_se[i] = hs ? 1 : 0;
         to_record(e, el[i]);
@@ -851,10 +1177,17 @@ int grid_for(uint64_t n, int block) {
 
 }  // namespace
 
-// Dynamic shared memory of transport_kernel: per thread, the leaf cache and
-// the event counters.
-static size_t transport_smem_bytes(int block) {
-    return size_t(kLeafCacheWords + kCounterSlots) * sizeof(float) * size_t(block);
+// Dynamic shared memory of a block: the transport kernel's pools, or the
+// sample kernel's leaf caches and event counters.
+static size_t transport_smem_bytes(int block, bool sample) {
+    return sample ? size_t(kLeafCacheWords + kCounterSlots) * sizeof(float) * size_t(block)
+                  : size_t(kWarpWords) * sizeof(uint32_t) * size_t(block / 32);
+}
+
+uint64_t transport_stack_bytes(int grid, int block, int depth, int mode) {
+    const uint64_t threads = uint64_t(grid) * uint64_t(block);
+    if (mode == kModeSample) return threads * 3 * sizeof(float4) * uint64_t(depth);
+    return threads / 32 * kStateWords * sizeof(uint32_t) * (32 * uint64_t(depth) + kDeepSlack);
 }
 
 // Shared-memory carveout that just fits the blocks the registers allow on an
@@ -864,7 +1197,7 @@ static size_t transport_smem_bytes(int block) {
 // size, device); the occupancy is checked afterwards and the default restored
 // if the hint would cost resident blocks.
 template <typename Kernel>
-static void fit_carveout(Kernel kernel, int block) {
+static void fit_carveout(Kernel kernel, int block, size_t dyn) {
     static std::mutex mu;
     static std::vector<std::pair<const void*, int>> done;
     int dev = 0;
@@ -875,9 +1208,15 @@ static void fit_carveout(Kernel kernel, int block) {
     for (const auto& d : done)
         if (d.first == key && d.second == tag) return;
     done.emplace_back(key, tag);
-    const size_t dyn = transport_smem_bytes(block);
     int before = 0, after = 0, smem_sm = 0;
     cudaFuncAttributes fa{};
+    // blocks that also hold the network exceed the 48 KB default; the largest
+    // block's need, whichever block size comes first
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(std::max(dyn, transport_smem_bytes(256, false)))) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&before, kernel, block, dyn) != cudaSuccess ||
         cudaFuncGetAttributes(&fa, kernel) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
@@ -899,64 +1238,51 @@ static void fit_carveout(Kernel kernel, int block) {
     }
 }
 
+// The kernel of a mode, model and variant (resident blocks per SM).
+using TransportKernel = void (*)(const dev::Physics, const TransportArgs);
 template <int Mode, bool Penn>
-static cudaError_t launch_mode(const dev::Physics& P, const TransportArgs& a, int grid, int block, int variant,
-                               cudaStream_t s) {
-    if (block <= 0 || block > (variant == 7 ? 128 : 256)) return cudaErrorInvalidValue;
-    const size_t sm = transport_smem_bytes(block);
-    switch (variant) {
-    case 2: fit_carveout(transport_kernel<2, Mode, Penn>, block); break;
-    case 4: fit_carveout(transport_kernel<4, Mode, Penn>, block); break;
-    case 7: fit_carveout(transport_kernel<7, Mode, Penn>, block); break;
-    default: fit_carveout(transport_kernel<3, Mode, Penn>, block); break;
+static TransportKernel kernel_of(int variant) {
+    if constexpr (Mode == kModeSample) {
+        return variant == 2 ? sample_kernel<2, Penn> : variant == 4 ? sample_kernel<4, Penn>
+             : variant == 7 ? sample_kernel<7, Penn> : sample_kernel<3, Penn>;
+    } else {
+        return variant == 2 ? transport_kernel<2, Mode, Penn> : variant == 4 ? transport_kernel<4, Mode, Penn>
+             : variant == 7 ? transport_kernel<7, Mode, Penn> : transport_kernel<3, Mode, Penn>;
     }
-    switch (variant) {
-    case 2: transport_kernel<2, Mode, Penn><<<grid, block, sm, s>>>(P, a); break;
-    case 4: transport_kernel<4, Mode, Penn><<<grid, block, sm, s>>>(P, a); break;
-    case 7: transport_kernel<7, Mode, Penn><<<grid, block, sm, s>>>(P, a); break;
-    default: transport_kernel<3, Mode, Penn><<<grid, block, sm, s>>>(P, a); break;
-    }
-    return cudaGetLastError();
 }
-
 template <bool Penn>
-static cudaError_t launch_model(const dev::Physics& P, const TransportArgs& a, int grid, int block, int variant,
-                                cudaStream_t s, int mode) {
-    if (mode == kModeSample) return launch_mode<kModeSample, Penn>(P, a, grid, block, variant, s);
-    if (mode == kModeLearned) return launch_mode<kModeLearned, Penn>(P, a, grid, block, variant, s);
-    if (mode == kModeDeposit) return launch_mode<kModeDeposit, Penn>(P, a, grid, block, variant, s);
-    if (mode == kModeWeighted) return launch_mode<kModeWeighted, Penn>(P, a, grid, block, variant, s);
-    return launch_mode<kModePlain, Penn>(P, a, grid, block, variant, s);
+static TransportKernel kernel_of(int mode, int variant) {
+    switch (mode) {
+    case kModeSample: return kernel_of<kModeSample, Penn>(variant);
+    case kModeLearned: return kernel_of<kModeLearned, Penn>(variant);
+    case kModeDeposit: return kernel_of<kModeDeposit, Penn>(variant);
+    case kModeWeighted: return kernel_of<kModeWeighted, Penn>(variant);
+    default: return kernel_of<kModePlain, Penn>(variant);
+    }
 }
 
 cudaError_t launch_transport(const dev::Physics& P, const TransportArgs& a, int grid, int block, int variant,
                              cudaStream_t s, int mode) {
-    return P.penn ? launch_model<true>(P, a, grid, block, variant, s, mode)
-                  : launch_model<false>(P, a, grid, block, variant, s, mode);
-}
-
-template <int Mode>
-static int max_blocks_mode(int block, int variant) {
-    int n = 0;
-    cudaError_t e;
-    const size_t sm = transport_smem_bytes(block);
-    switch (variant) {
-    // both models share launch bounds and shared memory, hence occupancy
-    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, transport_kernel<2, Mode, false>, block, sm); break;
-    case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, transport_kernel<4, Mode, false>, block, sm); break;
-    case 7: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, transport_kernel<7, Mode, false>, block, sm); break;
-    default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, transport_kernel<3, Mode, false>, block, sm); break;
-    }
-    if (e != cudaSuccess) return 1;
-    return n > 0 ? n : 1;
+    if (block <= 0 || block % 32 != 0 || block > (variant == 7 ? 128 : 256)) return cudaErrorInvalidValue;
+    if (mode == kModeSample && !a.stack_mem) return cudaErrorInvalidValue;
+    const TransportKernel kernel = P.penn ? kernel_of<true>(mode, variant) : kernel_of<false>(mode, variant);
+    const size_t sm = transport_smem_bytes(block, mode == kModeSample);
+    fit_carveout(kernel, block, sm);
+    kernel<<<grid, block, sm, s>>>(P, a);
+    return cudaGetLastError();
 }
 
 int transport_max_blocks_per_sm(int block, int variant, int mode) {
-    if (mode == kModeSample) return max_blocks_mode<kModeSample>(block, variant);
-    if (mode == kModeLearned) return max_blocks_mode<kModeLearned>(block, variant);
-    if (mode == kModeDeposit) return max_blocks_mode<kModeDeposit>(block, variant);
-    if (mode == kModeWeighted) return max_blocks_mode<kModeWeighted>(block, variant);
-    return max_blocks_mode<kModePlain>(block, variant);
+    int n = 0;
+    // both models share launch bounds and shared memory, hence occupancy
+    const TransportKernel kernel = kernel_of<false>(mode, variant);
+    const size_t sm = transport_smem_bytes(block, mode == kModeSample);
+    fit_carveout(kernel, block, sm);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, sm) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return n > 0 ? n : 1;
 }
 
 namespace {

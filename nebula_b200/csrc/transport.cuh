@@ -242,6 +242,23 @@ __device__ __forceinline__ bool in_domain(const Geometry& g, V3 p) {
            (p.z > g.cz - g.hz) && (p.z < g.cz + g.hz);
 }
 
+// True when the straight step of length `dist` from p (inside the domain)
+// along the unit vector d certainly meets no triangle, by the clearance map:
+// one 4-byte and at most one 16-byte gather.  NaN and infinities give false.
+__device__ __forceinline__ bool step_is_clear(const Clearance& m, V3 p, V3 d, float dist) {
+    if (!m.top) return false;
+    const int ix = int((p.x - m.lox) * m.inv_h), iy = int((p.y - m.loy) * m.inv_h), iz = int((p.z - m.loz) * m.inv_h);
+    const int top = __ldg(m.top + (size_t(iz >> 2) * m.ny + (iy >> 2)) * m.nx + (ix >> 2));
+    if (top < 0) return dist < (top == kClearFar ? m.far_reach : m.reach);
+    const float4 r = __ldg(m.rec + size_t(top) * 64 + ((iz & 3) * 16 + (iy & 3) * 4 + (ix & 3)));
+    // slab coordinate of both ends, relative to the fine cell's centre
+    const float qx = p.x - __fmaf_rn(float(ix) + 0.5f, m.h, m.lox), qy = p.y - __fmaf_rn(float(iy) + 0.5f, m.h, m.loy),
+                qz = p.z - __fmaf_rn(float(iz) + 0.5f, m.h, m.loz);
+    const float s0 = __fmaf_rn(r.x, qx, __fmaf_rn(r.y, qy, __fmaf_rn(r.z, qz, -r.w)));
+    const float s1 = __fmaf_rn(dist, __fmaf_rn(r.x, d.x, __fmaf_rn(r.y, d.y, r.z * d.z)), s0);
+    return dist < m.reach && (fminf(s0, s1) > 1.0f || fmaxf(s0, s1) < -1.0f);
+}
+
 // The octant offset (bit - 0.5) of geometry/octree.inl:65-67,79-81, as a
 // select: exactly +-0.5, without an integer-to-float conversion.
 __device__ __forceinline__ float half_step(unsigned bit) { return bit ? 0.5f : -0.5f; }
@@ -738,24 +755,19 @@ __device__ __forceinline__ bool ends_at_init(const Physics& P, const Electron& e
 }
 
 // One pass of init -> intersect -> scatter (drivers/cpu/cpu_driver.inl:73-161,
-// cpu_particle_manager.inl:214-235).  Uniforms of step k come from Philox
-// blocks (k, 0) and (k, 1) of the electron's stream: block 0 x/y feed the
-// inelastic/elastic free paths, z the ICDF probability (or the boundary
+// cpu_particle_manager.inl:214-235) in its three parts: free_path and
+// step_is_clear / propagate decide where the step ends, cross takes a step that
+// met a triangle, scatter one that did not.  Uniforms of step k come from
+// Philox blocks (k, 0) and (k, 1) of the electron's stream: block 0 x/y feed
+// the inelastic/elastic free paths, z the ICDF probability (or the boundary
 // transmission draw), w the scattering azimuth; block 1 the remaining four
-// inelastic draws.  The mechanisms' log(E) is the init pass's log(E): the
-// energy has not changed in between, so the value is the same.  kPenn
-// selects the inelastic model at compile time (P.penn must agree), as the
-// reference's physics_config.h does.
-template <bool kPenn>
-__device__ __forceinline__ int step(const Physics& P, Electron& e, int* event, Electron* se, bool* has_se,
-                                    LeafCache cache = LeafCache{nullptr, 0}) {
-    *event = kEvNone;
-    *has_se = false;
-    if (ends_at_init(P, e)) return kTerminated;
-    const uint4 r0 = draw(P.seed, e, 0);
-    int type = 0;
-    float dist = P.geo.max_extent;
-    float logE = 0;
+// inelastic draws.
+
+// Sampled path to the next event: *type 0 (vacuum: the domain's extent),
+// 1 inelastic or 2 elastic; r0 is the step's block 0.
+__device__ __forceinline__ void free_path(const Physics& P, const Electron& e, uint4 r0, int* type, float* dist) {
+    *type = 0;
+    *dist = P.geo.max_extent;
     if (e.mat >= 0) {
         const Material& m = P.mat[e.mat];
         // The free-path sampling uses the hardware log2/exp2 approximations
@@ -764,8 +776,8 @@ __device__ __forceinline__ int step(const Physics& P, Electron& e, int* event, E
         // are exact functions of the log E they are given.  A path that the
         // approximation would make slightly negative (U within 2^-21 of 1) is
         // taken as 0.
-        logE = __logf(e.E);
-        dist = __int_as_float(0x7f800000);
+        const float logE = __logf(e.E);
+        *dist = __int_as_float(0x7f800000);
         // Mean free path exp(-log imfp) rather than 1 / exp(log imfp): the
         // same exponential sampling (scatter_list.h:106-132, random.h
         // exponential) without a division per mechanism.
@@ -774,59 +786,95 @@ __device__ __forceinline__ int step(const Physics& P, Electron& e, int* event, E
         {
             const float mfp = __expf(-in_lg);
             const float path = fmaxf(-mfp * __logf(u01(r0.x)), 0.0f);
-            if (path < dist) {
-                type = 1;
-                dist = path;
+            if (path < *dist) {
+                *type = kEvInelastic;
+                *dist = path;
             }
         }
         {
             const float mfp = __expf(-el_lg);
             const float path = fmaxf(-mfp * __logf(u01(r0.y)), 0.0f);
-            if (path < dist) {
-                type = 2;
-                dist = path;
+            if (path < *dist) {
+                *type = kEvElastic;
+                *dist = path;
             }
         }
     }
-    const V3 nd = normalised(V3{e.dx, e.dy, e.dz});
-    int hit;
-    const float tdist = propagate(P.geo, V3{e.px, e.py, e.pz}, nd, dist, e.last_tri, e.mat, &hit, cache);
+}
+
+// The end of a step that met triangle `hit` after `t`, or (hit < 0) left the
+// domain in vacuum; rz is word z of the step's block 0.
+__device__ __forceinline__ int cross(const Physics& P, Electron& e, V3 nd, float t, int hit, uint32_t rz) {
+    e.px += nd.x * t;
+    e.py += nd.y * t;
+    e.pz += nd.z * t;
     int status = kAlive;
-    if (hit < 0) {
-        e.px += nd.x * dist;
-        e.py += nd.y * dist;
-        e.pz += nd.z * dist;
-        if (type != 0) {
-            // Shared first half of both mechanisms (see elastic_finish).
-            // Uniforms: block 0 z -> ICDF probability, w -> azimuth; block 1
-            // -> binding, energy loss and the two unit-vector draws.
-            e.last_tri = -1;
-            const Material& m = P.mat[e.mat];
-            const bool inel = (type == 1);
-            const float tv = table2d_get(inel ? m.in_icdf : m.el_icdf, logE, u01(r0.z));
-            const V3 n = approx::normalised(approx::make_normal_vec(nd, u01(r0.w)));
-            if (!inel) {
-                elastic_finish(m, e, tv, nd, n);
-                *event = kEvElastic;
-            } else {
-                const uint4 r1 = draw(P.seed, e, 1);
-                if constexpr (kPenn)
-                    *has_se = penn_finish(P, m, e, tv, logE, nd, n, r1, se);
-                else
-                    *has_se = inelastic_finish(m, e, tv, nd, n, u01(r1.x), u01(r1.y), u01(r1.z), u01(r1.w), se);
-                *event = kEvInelastic;
-            }
-        }
-    } else {
-        e.px += nd.x * tdist;
-        e.py += nd.y * tdist;
-        e.pz += nd.z * tdist;
+    if (hit >= 0) {
         e.last_tri = hit;
-        status = boundary(P, e, u01(r0.z));
-        *event = kEvBoundary;
+        status = boundary(P, e, u01(rz));
     }
     e.step += 1;
     return status;
+}
+
+// The scattering event (type 1 or 2) at the end of a step of length `dist`
+// along nd = normalised(direction); rz, rw are words z and w of the step's
+// block 0.  The mechanisms' log(E) is the init pass's: the energy has not
+// changed in between, so the value is the same.  kPenn selects the inelastic
+// model at compile time (P.penn must agree), as the reference's
+// physics_config.h does.
+template <bool kPenn>
+__device__ __forceinline__ void scatter(const Physics& P, Electron& e, V3 nd, float dist, int type, uint32_t rz,
+                                        uint32_t rw, Electron* se, bool* has_se) {
+    e.px += nd.x * dist;
+    e.py += nd.y * dist;
+    e.pz += nd.z * dist;
+    // Shared first half of both mechanisms (see elastic_finish).
+    // Uniforms: block 0 z -> ICDF probability, w -> azimuth; block 1
+    // -> binding, energy loss and the two unit-vector draws.
+    e.last_tri = -1;
+    const Material& m = P.mat[e.mat];
+    const bool inel = (type == kEvInelastic);
+    const float logE = __logf(e.E);
+    const float tv = table2d_get(inel ? m.in_icdf : m.el_icdf, logE, u01(rz));
+    const V3 n = approx::normalised(approx::make_normal_vec(nd, u01(rw)));
+    *has_se = false;
+    if (!inel) {
+        elastic_finish(m, e, tv, nd, n);
+    } else {
+        const uint4 r1 = draw(P.seed, e, 1);
+        if constexpr (kPenn)
+            *has_se = penn_finish(P, m, e, tv, logE, nd, n, r1, se);
+        else
+            *has_se = inelastic_finish(m, e, tv, nd, n, u01(r1.x), u01(r1.y), u01(r1.z), u01(r1.w), se);
+    }
+    e.step += 1;
+}
+
+// The whole pass for one electron.  kClear answers steps that cannot meet a
+// triangle from the clearance map (the same result as the walk: no hit).
+template <bool kPenn, bool kClear>
+__device__ __forceinline__ int step(const Physics& P, Electron& e, int* event, Electron* se, bool* has_se,
+                                    LeafCache cache = LeafCache{nullptr, 0}) {
+    *event = kEvNone;
+    *has_se = false;
+    if (ends_at_init(P, e)) return kTerminated;
+    const uint4 r0 = draw(P.seed, e, 0);
+    int type;
+    float dist;
+    free_path(P, e, r0, &type, &dist);
+    const V3 nd = normalised(V3{e.dx, e.dy, e.dz});
+    int hit = -1;
+    float t = dist;
+    if (!(kClear && type != 0 && step_is_clear(P.geo.clear, V3{e.px, e.py, e.pz}, nd, dist)))
+        t = propagate(P.geo, V3{e.px, e.py, e.pz}, nd, dist, e.last_tri, e.mat, &hit, cache);
+    if (hit >= 0 || type == 0) {
+        if (hit >= 0) *event = kEvBoundary;
+        return cross(P, e, nd, t, hit, r0.z);
+    }
+    *event = type;
+    scatter<kPenn>(P, e, nd, dist, type, r0.z, r0.w, se, has_se);
+    return kAlive;
 }
 
 }  // namespace dev

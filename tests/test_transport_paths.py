@@ -1,6 +1,9 @@
 """The transport's shortcuts against the general path they stand in for: the
 octree walk's plane rejection against the C restatement of octree::propagate,
-which tests every listed triangle."""
+which tests every listed triangle; and whole runs, whose steps skip the walk
+where the clearance map allows it and share a warp's electrons among its
+lanes, against the same cascades taken one nbx_step_query at a time, which
+walk every step."""
 import ctypes as C
 
 import numpy as np
@@ -70,3 +73,58 @@ def test_rays_match_the_walk_that_tests_every_triangle(name, inputs, ray_sampler
     assert (ot >= 0).sum() > n // 100
     assert np.array_equal(gt, ot)
     assert np.array_equal(gd.view(np.uint32), od.view(np.uint32))
+
+
+def cascades_step_by_step(ctx, prim, uid_base=0):
+    """Per-primary SE and BSE counts and the event totals (steps, inelastic,
+    elastic, boundary) of whole cascades, every electron advanced by single
+    general steps."""
+    import nebula_b200 as nb
+    n = len(prim)
+    e = np.zeros(n, nb.ELECTRON_DTYPE)
+    e["pos"], e["dir"], e["E"] = prim[:, 0:3], prim[:, 3:6], prim[:, 6]
+    e["mat"], e["last_tri"] = formats.VACUUM, -1
+    e["tag"], e["uid"] = np.arange(n), uid_base + np.arange(n)
+    se, bse, events = np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(4, np.int64)
+    while len(e):
+        e, st, ev, new, has = ctx.step_query(e)
+        events += [len(e)] + [(ev == k).sum() for k in (1, 2, 3)]
+        hit = e[st == 2]
+        np.add.at(se, hit["tag"][hit["E"] < 50], 1)
+        np.add.at(bse, hit["tag"][hit["E"] >= 50], 1)
+        e = np.concatenate([e[st == 0], new[has == 1]])
+    return se, bse, events
+
+
+def soup_in_a_block(seed=4):
+    """A block of material 0 with the sliver soup just below its top face:
+    arbitrary material changes, edges and needles in every cell."""
+    from nebula_b200 import generators as g
+    t = sliver_soup(seed, 600)
+    t["v"] *= np.float32(0.4)
+    t["v"][:, :, 2] -= np.float32(30.0)
+    t["mat_out"] = np.random.default_rng(seed).integers(0, 3, len(t))
+    return np.concatenate([g.cube_geometry(size=(300.0, 300.0, 200.0)), t])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("model", ["kieft", "penn"])
+@pytest.mark.parametrize("name", ["cube", "grating_small", "rough", "holes", "soup"])
+def test_run_equals_single_steps(name, model, inputs):
+    import nebula_b200 as nb
+    from nebula_b200 import generators as g
+    tris = soup_in_a_block() if name == "soup" else inputs[name]
+    top = {"cube": 1.0, "grating_small": 75.0, "rough": 20.0, "holes": 10.0, "soup": 1.0}[name]
+    recs = g.scan_beam(9, 9, 12, 500.0, spacing=8.0, origin=(-36.0, -36.0), z_start=top, seed=23,
+                       energies=[120.0, 500.0, 2000.0])
+    prim = np.concatenate([recs["pos"], recs["dir"], recs["E"][:, None]], 1).astype(np.float32)
+    ctx = nb.setup(tris, [inputs["si"], inputs["sio2"], inputs["w"]], device=0, seed=77, inelastic=model)
+    ctx.push(prim, np.arange(len(prim), dtype=np.uint32))
+    ctx.run()
+    s = ctx.stats()
+    got = ctx.tag_counts(0, len(prim))
+    se, bse, events = cascades_step_by_step(ctx, prim)
+    ctx.close()
+    assert events[1:].sum() > 20 * len(prim)
+    assert np.array_equal(got[0], se) and np.array_equal(got[1], bse)
+    assert [s[k] for k in ("steps", "events_inelastic", "events_elastic", "events_boundary")] == events.tolist()
