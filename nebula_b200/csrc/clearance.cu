@@ -8,19 +8,23 @@
 //
 // Layout: a coarse grid of cells over the octree's root box, each either
 // empty (nothing within `reach`, or within `far_reach`) or the index of a
-// brick of 4 x 4 x 4 records, one per fine cell of edge h.  A record is a
-// slab: every part of every triangle inside the fine cell's box, widened by
-// `reach` on all sides, lies within |n . q - c| <= 1, where q is the position
-// relative to the fine cell's centre and n the slab's normal divided by its
-// half thickness (a margin for rounding included).  A step shorter than
-// `reach` stays inside the widened box, so when both its ends lie on the same
-// side of the slab it meets no triangle.  One slab is enough: surfaces are
-// locally flat, so the slab is thin (only the margin, on flat faces).
+// brick of 4 x 4 x 4 records, one per fine cell of edge h.  A record is two
+// slabs: every part of every triangle inside the fine cell's box, widened by
+// `reach` on all sides, lies within |n . q - c| <= 1 of one of them, where q
+// is the position relative to the fine cell's centre and n the slab's normal
+// divided by its half thickness (a margin for rounding included).  A step
+// shorter than `reach` stays inside the widened box, so when its two ends lie
+// on the same side of the one slab and on the same side of the other it meets
+// no triangle.  Surfaces are locally flat, so a slab is thin (only the
+// margin, on flat faces); the second one serves edges and corners.
 //
-// h = 4 nm and reach = 3 nm: 99 % of the free paths are below 3 nm, and on
-// 20,000-step samples the share of steps answered was 0.84 (grating), 0.91
-// (rough slab) and 0.68 (contact holes); h = 2 gives 0.86 / 0.92 / 0.71 for
-// eight times the records, h = 8 with a reach of 8 nm 0.52 / 0.82 / 0.32.
+// h = 4 nm and reach = 3 nm: 99 % of the free paths are below 3 nm.  Share of
+// steps answered on 8,000-step samples (grating, rough slab, contact holes):
+// 0.92 / 0.91 / 0.83 with two slabs, 0.84 / 0.91 / 0.68 with one; h = 2 adds
+// 0.00 / 0.02 / 0.01 for eight times the records, h = 8 with a reach of 8 nm
+// and one slab gives 0.52 / 0.82 / 0.32.
+// B200, the second slab together with the walk's batched exact test: half the
+// benchmark's grating frame 98.2 -> 80.3 ms, contact holes 41.0 -> 30.4 ms.
 #include "clearance.h"
 
 #include <algorithm>
@@ -242,9 +246,24 @@ __device__ bool clipped_extent(float3 p0, float3 p1, float3 p2, float h, float3 
     return true;
 }
 
-// One block of 64 threads per brick, one thread per fine cell: the slab's
-// normal is the mean of the normals within 45 degrees of the nearest
-// candidate's, its extent that of all candidates' clipped parts.
+// One block of 64 threads per brick, one thread per fine cell.  The first slab
+// holds the candidates whose normals lie within 45 degrees of the nearest
+// one's, the second the others; each slab's normal is the mean of its
+// candidates' normals near that of its nearest, its extent that of its
+// candidates' clipped parts.
+__device__ __forceinline__ float3 unit_normal(const TriBox& t) {
+    const float nx = t.e1.y * t.e2.z - t.e1.z * t.e2.y, ny = t.e1.z * t.e2.x - t.e1.x * t.e2.z,
+                nz = t.e1.x * t.e2.y - t.e1.y * t.e2.x;
+    const float l2 = nx * nx + ny * ny + nz * nz;
+    const float s = l2 > 0.0f ? rsqrtf(l2) : 0.0f;
+    return make_float3(nx * s, ny * s, nz * s);
+}
+// +1 / -1: u lies within 45 degrees of n / of -n; 0: neither
+__device__ __forceinline__ float alike(float3 u, float3 n) {
+    const float d = u.x * n.x + u.y * n.y + u.z * n.z;
+    return d > 0.7f ? 1.0f : (d < -0.7f ? -1.0f : 0.0f);
+}
+
 __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const float4* tri, Grid g, const uint32_t* brick_cell,
                                                                          const uint64_t* start, const uint32_t* n_entry,
                                                                          const int32_t* entry, float margin, float4* rec) {
@@ -258,66 +277,73 @@ __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const 
     const float box = 0.5f * h + g.reach;
     const int32_t* list = entry + start[b];
     const int n = int(n_entry[b]);
-    float best = INFINITY;
-    int bi = -1;
-    for (int k = 0; k < n; ++k) {
-        const int t = __ldg(list + k);
-        if (!near_box(load_tri(tri, t), px, py, pz, box)) continue;
-        const float d2 = dev::dist2_to_triangle(tri, t, px, py, pz);
-        // (ties: the lowest index, so that the record does not depend on the list's order)
-        if (d2 < best || (d2 == best && t < bi) || bi < 0) {
-            best = d2;
-            bi = t;
-        }
-    }
-    float4 out = make_float4(0.0f, 0.0f, 0.0f, -2.0f);   // nothing near: n . q - c = 2 everywhere
-    if (bi >= 0) {
-        auto unit = [](const TriBox& t) {
-            const float nx = t.e1.y * t.e2.z - t.e1.z * t.e2.y, ny = t.e1.z * t.e2.x - t.e1.x * t.e2.z,
-                        nz = t.e1.x * t.e2.y - t.e1.y * t.e2.x;
-            const float l2 = nx * nx + ny * ny + nz * nz;
-            const float s = l2 > 0.0f ? rsqrtf(l2) : 0.0f;
-            return make_float3(nx * s, ny * s, nz * s);
-        };
-        const float3 n0 = unit(load_tri(tri, bi));
-        float sx = n0.x, sy = n0.y, sz = n0.z;
+    float3 first = make_float3(0.0f, 0.0f, 0.0f);   // normal that marks the first slab's candidates
+#pragma unroll 1
+    for (int slab = 0; slab < 2; ++slab) {
+        // this slab's nearest candidate
+        float best = INFINITY;
+        int bi = -1;
         for (int k = 0; k < n; ++k) {
             const int t = __ldg(list + k);
-            if (t == bi) continue;
             const TriBox tb = load_tri(tri, t);
-            if (!near_box(tb, px, py, pz, box)) continue;
-            const float3 u = unit(tb);
-            const float d = u.x * n0.x + u.y * n0.y + u.z * n0.z;
-            const float s = d > 0.7f ? 1.0f : (d < -0.7f ? -1.0f : 0.0f);
-            sx += s * u.x;
-            sy += s * u.y;
-            sz += s * u.z;
-        }
-        float l2 = sx * sx + sy * sy + sz * sz;
-        if (!(l2 > 1e-12f)) {   // no usable normal (degenerate triangles): any direction serves
-            sx = sy = 0.0f;
-            sz = l2 = 1.0f;
-        }
-        const float s = rsqrtf(l2);
-        const float3 u = make_float3(sx * s, sy * s, sz * s);
-        float lo = INFINITY, hi = -INFINITY;
-        for (int k = 0; k < n; ++k) {
-            const TriBox tb = load_tri(tri, __ldg(list + k));
-            if (!near_box(tb, px, py, pz, box)) continue;
-            const float3 p0 = make_float3(tb.a.x - px, tb.a.y - py, tb.a.z - pz);
-            float a, e;
-            if (clipped_extent(p0, make_float3(p0.x + tb.e1.x, p0.y + tb.e1.y, p0.z + tb.e1.z),
-                               make_float3(p0.x + tb.e2.x, p0.y + tb.e2.y, p0.z + tb.e2.z), box, u, a, e)) {
-                lo = fminf(lo, a);
-                hi = fmaxf(hi, e);
+            if (!near_box(tb, px, py, pz, box) || (slab == 1 && alike(unit_normal(tb), first) != 0.0f)) continue;
+            const float d2 = dev::dist2_to_triangle(tri, t, px, py, pz);
+            // (ties: the lowest index, so that the record does not depend on the list's order)
+            if (d2 < best || (d2 == best && t < bi) || bi < 0) {
+                best = d2;
+                bi = t;
             }
         }
-        if (hi >= lo) {
-            const float inv = 1.0f / (0.5f * (hi - lo) + margin);
-            out = make_float4(u.x * inv, u.y * inv, u.z * inv, 0.5f * (hi + lo) * inv);
+        float4 out = make_float4(0.0f, 0.0f, 0.0f, -2.0f);   // nothing near: n . q - c = 2 everywhere
+        if (bi >= 0) {
+            float3 u = unit_normal(load_tri(tri, bi));
+            // a first slab without a normal (zero area) takes every candidate
+            const bool all = slab == 0 && u.x == 0.0f && u.y == 0.0f && u.z == 0.0f;
+            const float3 near = u;
+            if (slab == 0) first = near;
+            float sx = 0.0f, sy = 0.0f, sz = 0.0f;
+            for (int k = 0; k < n; ++k) {
+                const TriBox tb = load_tri(tri, __ldg(list + k));
+                if (!near_box(tb, px, py, pz, box)) continue;
+                const float3 v = unit_normal(tb);
+                if (slab == 1 && alike(v, first) != 0.0f) continue;
+                const float s = alike(v, near);
+                sx += s * v.x;
+                sy += s * v.y;
+                sz += s * v.z;
+            }
+            float l2 = sx * sx + sy * sy + sz * sz;
+            if (!(l2 > 1e-12f)) {   // no usable normal (degenerate triangles): any direction serves
+                sx = sy = 0.0f;
+                sz = l2 = 1.0f;
+            }
+            const float s = rsqrtf(l2);
+            u = make_float3(sx * s, sy * s, sz * s);
+            float lo = INFINITY, hi = -INFINITY;
+            for (int k = 0; k < n; ++k) {
+                const TriBox tb = load_tri(tri, __ldg(list + k));
+                if (!near_box(tb, px, py, pz, box)) continue;
+                if (!all && (alike(unit_normal(tb), first) != 0.0f) != (slab == 0)) continue;
+                const float3 p0 = make_float3(tb.a.x - px, tb.a.y - py, tb.a.z - pz);
+                float a, e;
+                if (clipped_extent(p0, make_float3(p0.x + tb.e1.x, p0.y + tb.e1.y, p0.z + tb.e1.z),
+                                   make_float3(p0.x + tb.e2.x, p0.y + tb.e2.y, p0.z + tb.e2.z), box, u, a, e)) {
+                    lo = fminf(lo, a);
+                    hi = fmaxf(hi, e);
+                }
+            }
+            if (hi >= lo) {
+                const float inv = 1.0f / (0.5f * (hi - lo) + margin);
+                out = make_float4(u.x * inv, u.y * inv, u.z * inv, 0.5f * (hi + lo) * inv);
+            }
+            if (all) {   // nothing is left for the second slab
+                rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i)] = out;
+                rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i) + 1] = make_float4(0.0f, 0.0f, 0.0f, -2.0f);
+                return;
+            }
         }
+        rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i) + slab] = out;
     }
-    rec[size_t(b) * (kBrick * kBrick * kBrick) + i] = out;
 }
 
 template <typename T>
@@ -351,7 +377,7 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
                      ClearanceMap* out) {
     constexpr float kFineCell = 4.0f, kReach = 3.0f;
     constexpr uint64_t kMaxCells = 1ull << 26, kMaxRecordBytes = 4ull << 30;
-    constexpr uint64_t kBrickCells = kBrick * kBrick * kBrick;
+    constexpr uint64_t kBrickCells = kBrick * kBrick * kBrick, kRecordBytes = 2 * sizeof(float4);
     float scale = 0.0f;   // largest coordinate: sizes the rounding margin
     for (int i = 0; i < 3; ++i) {
         if (!(half[i] > 0.0f) || !(half[i] < 1e18f) || !(std::fabs(center[i]) < 1e18f)) return false;
@@ -403,12 +429,12 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
             cudaMemcpyAsync(used, totals.p, 16, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess)
             return false;
-        if (used[0] * kBrickCells * sizeof(float4) > budget || used[1] * 4 > budget) continue;
+        if (used[0] * kBrickCells * kRecordBytes > budget || used[1] * 4 > budget) continue;
         Temp<int32_t> top, entry;
         Temp<float4> rec;
         Temp<uint64_t> start;
         Temp<uint32_t> brick_cell, cursor;
-        if (!top.alloc(cells) || !entry.alloc(used[1]) || !rec.alloc(used[0] * kBrickCells) || !start.alloc(used[0]) ||
+        if (!top.alloc(cells) || !entry.alloc(used[1]) || !rec.alloc(used[0] * kBrickCells * 2) || !start.alloc(used[0]) ||
             !brick_cell.alloc(used[0]) || !cursor.alloc(used[0]) ||
             cudaMemsetAsync(cursor.p, 0, 4 * std::max<uint64_t>(used[0], 1), s) != cudaSuccess)
             return false;

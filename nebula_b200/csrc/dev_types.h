@@ -49,7 +49,7 @@ struct Material {
 // Clearance map (clearance.cu): a coarse grid (nx x ny x ..., x fastest) over
 // the octree's root box whose cells are empty (kClearNear: no triangle within
 // `reach`, kClearFar: none within `far_reach`) or index a brick of 4 x 4 x 4
-// slab records (n, c), one per fine cell of edge h.
+// records of two slabs (n, c), one record per fine cell of edge h.
 constexpr int kClearNear = -1, kClearFar = -2;
 struct Clearance {
     const int* top;           // nullptr: no map

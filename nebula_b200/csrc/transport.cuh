@@ -201,15 +201,6 @@ __device__ __forceinline__ V3 make_unit_vec(float cos_theta, float u_phi) {
 // ---------------------------------------------------------------------------
 // Geometry
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void load_tri_vertices(const Geometry& g, int ti, V3& r0, V3& e1, V3& e2) {
-    const float4 a = __ldg(g.tri + 3 * ti);
-    const float4 b = __ldg(g.tri + 3 * ti + 1);
-    const float4 c = __ldg(g.tri + 3 * ti + 2);
-    r0 = {a.x, a.y, a.z};
-    e1 = {b.x, b.y, b.z};
-    e2 = {c.x, c.y, c.z};
-}
-
 // Unnormalised normal e1 x e2 (triangle::get_normal, core/triangle.inl:71-74)
 // and the two materials, from the triangle's 16-byte face record.
 __device__ __forceinline__ V3 load_face(const Geometry& g, int ti, int& mi, int& mo) {
@@ -244,19 +235,23 @@ __device__ __forceinline__ bool in_domain(const Geometry& g, V3 p) {
 
 // True when the straight step of length `dist` from p (inside the domain)
 // along the unit vector d certainly meets no triangle, by the clearance map:
-// one 4-byte and at most one 16-byte gather.  NaN and infinities give false.
+// one 4-byte gather and at most one of 32 bytes.  Infinite paths give false.
 __device__ __forceinline__ bool step_is_clear(const Clearance& m, V3 p, V3 d, float dist) {
     if (!m.top) return false;
     const int ix = int((p.x - m.lox) * m.inv_h), iy = int((p.y - m.loy) * m.inv_h), iz = int((p.z - m.loz) * m.inv_h);
     const int top = __ldg(m.top + (size_t(iz >> 2) * m.ny + (iy >> 2)) * m.nx + (ix >> 2));
     if (top < 0) return dist < (top == kClearFar ? m.far_reach : m.reach);
-    const float4 r = __ldg(m.rec + size_t(top) * 64 + ((iz & 3) * 16 + (iy & 3) * 4 + (ix & 3)));
-    // slab coordinate of both ends, relative to the fine cell's centre
+    const float4* const rec = m.rec + 2 * (size_t(top) * 64 + ((iz & 3) * 16 + (iy & 3) * 4 + (ix & 3)));
+    const float4 r = __ldg(rec), t = __ldg(rec + 1);
+    // slab coordinates of both ends, relative to the fine cell's centre
     const float qx = p.x - __fmaf_rn(float(ix) + 0.5f, m.h, m.lox), qy = p.y - __fmaf_rn(float(iy) + 0.5f, m.h, m.loy),
                 qz = p.z - __fmaf_rn(float(iz) + 0.5f, m.h, m.loz);
     const float s0 = __fmaf_rn(r.x, qx, __fmaf_rn(r.y, qy, __fmaf_rn(r.z, qz, -r.w)));
     const float s1 = __fmaf_rn(dist, __fmaf_rn(r.x, d.x, __fmaf_rn(r.y, d.y, r.z * d.z)), s0);
-    return dist < m.reach && (fminf(s0, s1) > 1.0f || fmaxf(s0, s1) < -1.0f);
+    const float t0 = __fmaf_rn(t.x, qx, __fmaf_rn(t.y, qy, __fmaf_rn(t.z, qz, -t.w)));
+    const float t1 = __fmaf_rn(dist, __fmaf_rn(t.x, d.x, __fmaf_rn(t.y, d.y, t.z * d.z)), t0);
+    return dist < m.reach && fminf(fabsf(s0), fabsf(s1)) > 1.0f && (s0 < 0.0f) == (s1 < 0.0f) &&
+           fminf(fabsf(t0), fabsf(t1)) > 1.0f && (t0 < 0.0f) == (t1 < 0.0f);
 }
 
 // The octant offset (bit - 0.5) of geometry/octree.inl:65-67,79-81, as a
@@ -390,28 +385,41 @@ __device__ __forceinline__ float propagate(const Geometry& g, V3 start, V3 dir, 
                 target = -4;
             }
         }
-        for (;;) {
-            const int ti = __ldg(od + index);
-            ++index;
-            if (ti < 0) break;
-            if (ti == ignore_tri) continue;
+        // The leaf's triangles, up to 32 at a time: first the plane test of
+        // all, then the exact test of those it leaves, in list order.  Lanes
+        // find their few survivors at different places of their lists; taken
+        // in a loop of their own the lanes test them together (a walk of 32
+        // lanes ran 5-8 rounds of the exact test for 0.9 survivors a lane).
+        for (bool more = true; more;) {
             // A triangle beyond both the best candidate so far and the rest
             // of the path cannot change the answer: an intersection past
             // to_go only ever replaces another one past to_go.
-            if (plane_misses(g, ti, cur, dir, fminf(intersect, to_go))) continue;
-            // The face record alone decides the exit material (the normal is
-            // e1 x e2 as computed on the device, so the sign is the
-            // reference's); only candidates that survive load the vertices.
-            int mi, mo;
-            const V3 nrm = load_face(g, ti, mi, mo);
-            const int mat_out = (dot(nrm, dir) < 0) ? mi : mo;
-            if (mat_out == ignore_mat) continue;
-            V3 r0, e1, e2;
-            load_tri_vertices(g, ti, r0, e1, e2);
-            const float t = intersect_ray(r0, e1, e2, cur, dir);
-            if ((t > 0) && (t <= intersect + kEps)) {
-                intersect = t;
-                target = ti;
+            const float bound = fminf(intersect, to_go);
+            const int first = index;
+            unsigned left = 0;
+            int ti = __ldg(od + index);
+            while (ti >= 0 && index - first < 32) {
+                const int next = __ldg(od + index + 1);   // ti is no terminator, so there is one
+                if (ti != ignore_tri && !plane_misses(g, ti, cur, dir, bound)) left |= 1u << (index - first);
+                ++index;
+                ti = next;
+            }
+            more = ti >= 0;
+            while (left) {
+                const int k = __ffs(left) - 1;
+                left &= left - 1;
+                const int tk = __ldg(od + first + k);
+                const float4 A = __ldg(g.tri + 3 * tk), B = __ldg(g.tri + 3 * tk + 1), C = __ldg(g.tri + 3 * tk + 2);
+                const V3 r0{A.x, A.y, A.z}, e1{B.x, B.y, B.z}, e2{C.x, C.y, C.z};
+                // the side decides the exit material (normal e1 x e2,
+                // core/triangle.inl:71-74)
+                const int mat_out = (dot(cross(e1, e2), dir) < 0) ? __float_as_int(A.w) : __float_as_int(B.w);
+                if (mat_out == ignore_mat) continue;
+                const float t = intersect_ray(r0, e1, e2, cur, dir);
+                if ((t > 0) && (t <= intersect + kEps)) {
+                    intersect = t;
+                    target = tk;
+                }
             }
         }
         if (intersect >= to_go) {
