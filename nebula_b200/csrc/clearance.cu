@@ -409,7 +409,9 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         g.loz = center[2] - half[2];
         double dims[3];
         for (int i = 0; i < 3; ++i) dims[i] = std::ceil(2.0 * double(half[i]) / double(g.cell)) + 1.0;
-        if (dims[0] * dims[1] * dims[2] > double(kMaxCells)) continue;
+        // (below 2^22 fine cells an axis: the transport's index arithmetic)
+        if (dims[0] * dims[1] * dims[2] > double(kMaxCells) || std::max({dims[0], dims[1], dims[2]}) > double(1 << 19))
+            continue;
         g.nx = int(dims[0]);
         g.ny = int(dims[1]);
         g.nz = int(dims[2]);
@@ -454,9 +456,12 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         dev::Clearance& m = out->map;
         m.top = out->top;
         m.rec = out->rec;
-        m.lox = g.lox;
-        m.loy = g.loy;
-        m.loz = g.loz;
+        m.offx = float(-double(g.lox) / fine - 0.5);
+        m.offy = float(-double(g.loy) / fine - 0.5);
+        m.offz = float(-double(g.loz) / fine - 0.5);
+        m.midx = g.lox + 0.5f * fine;
+        m.midy = g.loy + 0.5f * fine;
+        m.midz = g.loz + 0.5f * fine;
         m.h = fine;
         m.inv_h = 1.0f / fine;
         m.nx = g.nx;

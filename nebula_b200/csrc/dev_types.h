@@ -36,6 +36,7 @@ struct Table3D {
 // rebuilt 2-D ionisation table, q and ion3 the full Penn 3-D tables.
 struct Material {
     float barrier;
+    float e_min, e_max;   // barrier + the run's energy limits
     float phonon_loss, recoil_const;
     float fermi, band_gap;
     Table1D el_imfp, in_imfp;
@@ -54,7 +55,8 @@ constexpr int kClearNear = -1, kClearFar = -2;
 struct Clearance {
     const int* top;           // nullptr: no map
     const float4* rec;
-    float lox, loy, loz;
+    float offx, offy, offz;   // -corner / h - 1/2
+    float midx, midy, midz;   // centre of fine cell (0, 0, 0)
     float h, inv_h;
     int nx, ny;
     float reach, far_reach;
@@ -67,6 +69,7 @@ struct Geometry {
     const float4* tri_plane;  // per triangle: (n, n . r0), n the normal of length 1 / rounding margin (nm)
     Clearance clear;
     float cx, cy, cz, hx, hy, hz;
+    float lox, loy, loz, hix, hiy, hiz;   // centre -+ half size
     float max_extent;
     int n_tri;
 };

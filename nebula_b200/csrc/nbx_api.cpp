@@ -640,6 +640,12 @@ int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* o) {
         g.hx = o->halfsize[0];
         g.hy = o->halfsize[1];
         g.hz = o->halfsize[2];
+        g.lox = g.cx - g.hx;
+        g.loy = g.cy - g.hy;
+        g.loz = g.cz - g.hz;
+        g.hix = g.cx + g.hx;
+        g.hiy = g.cy + g.hy;
+        g.hiz = g.cz + g.hz;
         // octree factory: 2 * magnitude(halfsize), host sqrt (geometry/octree.inl:247-253)
         g.max_extent = 2 * std::sqrt(g.hx * g.hx + g.hy * g.hy + g.hz * g.hz);
         g.n_tri = int(o->n_triangles);
@@ -684,6 +690,10 @@ int nbx_add_material(nbx_ctx* ctx, const nbx_material* m) {
         // cpu_material_manager::get_max_energy (core/cpu_material_manager.inl:43-55)
         if (max_energy < ctx->max_energy) ctx->max_energy = max_energy;
         ctx->phys.max_energy = ctx->max_energy;
+        for (nbx::dev::Material& x : ctx->phys.mat) {
+            x.e_min = x.barrier + ctx->phys.min_energy;
+            x.e_max = x.barrier + ctx->phys.max_energy;
+        }
         return NBX_OK;
     });
 }
