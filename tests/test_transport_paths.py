@@ -128,3 +128,34 @@ def test_run_equals_single_steps(name, model, inputs):
     assert events[1:].sum() > 20 * len(prim)
     assert np.array_equal(got[0], se) and np.array_equal(got[1], bse)
     assert [s[k] for k in ("steps", "events_inelastic", "events_elastic", "events_boundary")] == events.tolist()
+
+
+@pytest.mark.gpu
+def test_table_indices_at_the_edges(inputs):
+    """Table lookups whose index is clamped: below and above the axes, on
+    every grid point and its neighbours, huge, infinite and NaN coordinates
+    (the restatement's floor-to-int turns the last three into index 0)."""
+    import ctypes as C
+    import nebula_b200 as nb
+    import oracle
+    m = nb.HostMaterial(inputs["si"])
+    ctx = nb.Context(device=0)
+    ctx.add_material(m)
+    P = oracle.port()
+    for name in ("el_imfp", "in_imfp", "el_icdf", "in_icdf", "ion"):
+        a, (x0, xs, y0, ys) = m.tables[name]
+        a = np.ascontiguousarray(a, np.float32)
+        grid = np.float32(x0) + np.arange(a.shape[0], dtype=np.float32) / np.float32(xs)
+        x = np.concatenate([grid, np.nextafter(grid, np.float32(-np.inf)), np.nextafter(grid, np.float32(np.inf)),
+                            np.array([-1e30, -5, 5e9, 1e30, np.inf, -np.inf, np.nan], np.float32)]).astype(np.float32)
+        y = np.resize(np.array([0.0, 1e-7, 0.5, 0.9999999, 1.0, -0.25, 1.75, 1e12], np.float32), len(x))
+        got = ctx.table_query(0, name, x, y)
+        if name.endswith("imfp"):
+            t = oracle.Table1D(len(a), x0, xs, a.ctypes.data)
+            want = [P.nbo_table1d_get(C.byref(t), float(v)) for v in x]
+        else:
+            t = oracle.Table2D(a.shape[0], a.shape[1], x0, xs, y0, ys, a.ctypes.data)
+            f = P.nbo_table2d_get_rounddown if name == "ion" else P.nbo_table2d_get
+            want = [f(C.byref(t), float(v), float(w)) for v, w in zip(x, y)]
+        assert np.array_equal(got, np.array(want, np.float32), equal_nan=True), name
+    ctx.close()
