@@ -203,8 +203,14 @@ int run_transport_noalloc(const dev::Physics& P, int grid, int block, int varian
                           uint64_t n_tags, uint64_t counts[4], const char** err);
 cudaError_t launch_fill_queue(Queue q, const float* particles, const uint32_t* tags, uint64_t uid_base,
                               uint64_t n, uint64_t offset, cudaStream_t s);
-// *p = v on the device, in stream order.
-cudaError_t launch_set_word(uint32_t* p, uint32_t v, cudaStream_t s);
+// A run's control block: zeroes `words` control words and the pop cursors,
+// then *n_queued = n and *overflow_before = *overflow.
+cudaError_t launch_begin_run(uint32_t* ctl, uint32_t words, uint32_t* cursors, uint32_t n_cursors, uint32_t* n_queued,
+                             uint32_t n, unsigned long long* overflow_before, const unsigned long long* overflow,
+                             cudaStream_t s);
+// report = {*tail, *overflow - *overflow_before}.
+cudaError_t launch_report_run(const uint32_t* tail, const unsigned long long* overflow_before,
+                              const unsigned long long* overflow, unsigned long long* report, cudaStream_t s);
 // The largest of n tags into *out (which the caller zeroes first).
 cudaError_t launch_max_tag(const uint32_t* tags, uint64_t n, uint32_t* out, cudaStream_t s);
 

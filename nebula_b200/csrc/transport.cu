@@ -15,6 +15,7 @@
 #include <cooperative_groups/reduce.h>
 
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -1151,9 +1152,27 @@ __global__ void fill_queue_kernel(Queue q, const float* particles, const uint32_
     }
 }
 
-// One word set on the device: a run's queue length goes into its control
-// block this way rather than by a host-to-device copy, which could wait
-// behind a staged batch's copy on the same copy engine.
+// A run's control block, prepared and read back by kernels: one small launch
+// in place of memsets and copies, which could also wait behind a staged
+// batch's copy on the same copy engine.  Zeroes `words` control words and the
+// pop cursors, sets the queue length and takes down the overflow counter.
+__global__ void begin_run_kernel(uint32_t* ctl, uint32_t words, uint32_t* cursors, uint32_t n_cursors, uint32_t* n_queued,
+                                 uint32_t n, unsigned long long* overflow_before, const unsigned long long* overflow) {
+    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) ctl[i] = 0u;
+    for (uint32_t i = threadIdx.x; i < n_cursors; i += blockDim.x) cursors[i] = 0u;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *n_queued = n;
+        *overflow_before = *overflow;
+    }
+}
+// For the host, side by side: the size of the last generation's output queue
+// and the electrons lost in this run.
+__global__ void report_run_kernel(const uint32_t* tail, const unsigned long long* overflow_before,
+                                  const unsigned long long* overflow, unsigned long long* report) {
+    report[0] = *tail;
+    report[1] = *overflow - *overflow_before;
+}
 __global__ void set_word_kernel(uint32_t* p, uint32_t v) { *p = v; }
 
 // Largest of n tags into *out (zeroed by the caller).
@@ -1407,8 +1426,16 @@ cudaError_t launch_pixel_yields(const uint32_t* se, const uint32_t* bse, const f
     return cudaGetLastError();
 }
 
-cudaError_t launch_set_word(uint32_t* p, uint32_t v, cudaStream_t s) {
-    set_word_kernel<<<1, 1, 0, s>>>(p, v);
+cudaError_t launch_begin_run(uint32_t* ctl, uint32_t words, uint32_t* cursors, uint32_t n_cursors, uint32_t* n_queued,
+                             uint32_t n, unsigned long long* overflow_before, const unsigned long long* overflow,
+                             cudaStream_t s) {
+    begin_run_kernel<<<1, 1024, 0, s>>>(ctl, words, cursors, n_cursors, n_queued, n, overflow_before, overflow);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_report_run(const uint32_t* tail, const unsigned long long* overflow_before,
+                              const unsigned long long* overflow, unsigned long long* report, cudaStream_t s) {
+    report_run_kernel<<<1, 1, 0, s>>>(tail, overflow_before, overflow, report);
     return cudaGetLastError();
 }
 
@@ -1502,7 +1529,8 @@ int run_transport_noalloc(const dev::Physics& P, int grid, int block, int varian
         return cudaStreamSynchronize(s) == cudaSuccess ? 0 : fail("stream synchronisation failed");
     }
     const uint32_t n_prim = n;
-    if (launch_set_word(ctl + 2 * kNoAllocGenerations, n_prim, s) != cudaSuccess)
+    set_word_kernel<<<1, 1, 0, s>>>(ctl + 2 * kNoAllocGenerations, n_prim);
+    if (cudaGetLastError() != cudaSuccess)
         return fail("writing the primary count failed");
     fill_queue_kernel<<<grid_for(n, 256), 256, 0, s>>>(prim, d_particles, d_tags, uid_base, n, 0);
     if (cudaGetLastError() != cudaSuccess) return fail("queue fill launch failed");
@@ -1513,9 +1541,15 @@ int run_transport_noalloc(const dev::Physics& P, int grid, int block, int varian
     a.n_tags = n_tags;
     a.counters = cnt;
     a.out_capacity = uint32_t(kNoAllocOverflow);
+    // The first generation's launch is checked by itself: with a warp's stack
+    // nearly every run ends there.  One copy brings the output queue's size and
+    // the counters, which follow it in the scratch.
+    constexpr size_t kReportBytes = kNoAllocScratchBytes - (kOffCtl + sizeof(uint32_t) * kNoAllocGenerations);
+    alignas(8) unsigned char report[kReportBytes];
     int g = 0;
     for (;;) {
-        for (int k = 0; k < 8 && g < kNoAllocGenerations; ++k, ++g) {
+        const int chunk = g == 0 ? 1 : 8;
+        for (int k = 0; k < chunk && g < kNoAllocGenerations; ++k, ++g) {
             a.in = g == 0 ? prim : ov[(g - 1) % 2];
             a.in_capacity = uint32_t(g == 0 ? kNoAllocMaxPrimaries : kNoAllocOverflow);
             a.out = ov[g % 2];
@@ -1524,10 +1558,11 @@ int run_transport_noalloc(const dev::Physics& P, int grid, int block, int varian
             a.out_tail = ctl + kNoAllocGenerations + g;
             if (launch_transport(P, a, grid, block, variant, s) != cudaSuccess) return fail("transport launch failed");
         }
-        uint32_t last = 0;
-        if (cudaMemcpyAsync(&last, ctl + kNoAllocGenerations + (g - 1), 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        if (cudaMemcpyAsync(report, ctl + kNoAllocGenerations, kReportBytes, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess)
             return fail("transport failed");
+        uint32_t last = 0;
+        std::memcpy(&last, report + sizeof(uint32_t) * (g - 1), sizeof(last));
         if (last == 0) break;
         if (g >= kNoAllocGenerations) {
             *err = "secondary generations exceed the allocation-free limit";
@@ -1535,8 +1570,7 @@ int run_transport_noalloc(const dev::Physics& P, int grid, int block, int varian
         }
     }
     unsigned long long c[kNumCounters];
-    if (cudaMemcpyAsync(c, cnt, sizeof(c), cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
-        return fail("reading counters failed");
+    std::memcpy(c, report + (kOffCnt - kOffCtl - sizeof(uint32_t) * kNoAllocGenerations), sizeof(c));
     if (counts) {
         counts[0] = c[kCntElastic];
         counts[1] = c[kCntInelastic];
