@@ -196,6 +196,8 @@ constexpr int kWarpWords = kRing * kWalkWords + kTop * kStateWords;
 // and the ones that queue up meanwhile: 24 keeps the walk's lanes mostly full
 // and leaves room.
 constexpr int kWalkBatch = 24;
+// Primaries a warp takes at a time.
+constexpr uint32_t kAsk = 4;
 // Ring codes: the scattering event that waits (1 inelastic, 2 elastic, as in
 // the walk's input; 0: none, the step starts in vacuum), an electron whose next
 // step starts, one that ended.
@@ -458,7 +460,9 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
         // Every electron a lane holds here is about to start a step.
         if (n_wait > 0 && n_back == 0) {
             const bool other_work = !drained || top_n + deep_n > 0;
-            if (n_wait >= kWalkBatch || (!other_work && n_wait >= __popc(__ballot_sync(kFull, have)))) walk();
+            // (at the end, waiting electrons go before twice as many running
+            // ones: a chain of steps is what the warp's time depends on then)
+            if (n_wait >= kWalkBatch || (!other_work && 2 * n_wait >= __popc(__ballot_sync(kFull, have)))) walk();
         }
         // -- idle lanes take work: back from the walk, then parked, then a
         // primary
@@ -505,9 +509,11 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
                 }
                 const int open = want - n1 - n2;
                 if (open > 0 && deep_n == 0 && !drained) {
-                    // Primaries: all open lanes' worth while the range holds
-                    // plenty, a warp's share of what is left toward its end
-                    // (so a small batch spreads over the warps).
+                    // Primaries: a few at a time, fewer toward the range's
+                    // end.  Their cascades fill the lanes, and what a warp has
+                    // not taken yet another one can take: with all open lanes'
+                    // worth at once, a contact-hole scan whose plugs scatter
+                    // more than its film ended at 22.8 ms instead of 16.5.
                     uint32_t lo = 0, len = n_in;
                     uint32_t* cursor = a.head;
                     if (a.range_cursor) {
@@ -519,7 +525,7 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
                         len = uint32_t(uint64_t(n_in) * (v + 1) / a.n_ranges) - lo;
                         cursor = a.range_cursor + v;
                     }
-                    const uint32_t ask = min(uint32_t(open), max(1u, (len - min(taken, len)) >> warps_log2));
+                    const uint32_t ask = min(min(uint32_t(open), kAsk), max(1u, (len - min(taken, len)) >> warps_log2));
                     uint32_t base = 0;
                     if (lane == 0) base = atomicAdd(cursor, ask);
                     base = __shfl_sync(kFull, base, 0);
