@@ -208,8 +208,18 @@ __global__ void __launch_bounds__(256) assign_kernel(const uint32_t* count, Grid
 }
 
 // Extent along n of the part of a triangle inside the box of half edge h
-// round the origin (Sutherland-Hodgman clipping); false when there is none.
-__device__ bool clipped_extent(float3 p0, float3 p1, float3 p2, float h, float3 n, float& lo, float& hi) {
+// round the origin; false when there is none.  A triangle that lies in the
+// box, or whose extent along n is next to nothing anyway (a flat face under
+// its own normal), counts whole; the others are clipped (Sutherland-Hodgman,
+// in local memory: on a flat geometry it was most of the map's time).
+__device__ bool clipped_extent(float3 p0, float3 p1, float3 p2, float h, float3 n, float flat, float& lo, float& hi) {
+    const float d0 = n.x * p0.x + n.y * p0.y + n.z * p0.z, d1 = n.x * p1.x + n.y * p1.y + n.z * p1.z,
+                d2 = n.x * p2.x + n.y * p2.y + n.z * p2.z;
+    lo = min3(d0, d1, d2);
+    hi = max3(d0, d1, d2);
+    const float reach = max3(max3(fabsf(p0.x), fabsf(p0.y), fabsf(p0.z)), max3(fabsf(p1.x), fabsf(p1.y), fabsf(p1.z)),
+                             max3(fabsf(p2.x), fabsf(p2.y), fabsf(p2.z)));
+    if (reach <= h || hi - lo <= flat) return true;
     // a convex polygon gains at most one vertex per plane (nine in all); one
     // that rounding has folded could gain more, and keeps what it has then
     // (clipping less only widens the extent)
@@ -327,7 +337,8 @@ __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const 
                 const float3 p0 = make_float3(tb.a.x - px, tb.a.y - py, tb.a.z - pz);
                 float a, e;
                 if (clipped_extent(p0, make_float3(p0.x + tb.e1.x, p0.y + tb.e1.y, p0.z + tb.e1.z),
-                                   make_float3(p0.x + tb.e2.x, p0.y + tb.e2.y, p0.z + tb.e2.z), box, u, a, e)) {
+                                   make_float3(p0.x + tb.e2.x, p0.y + tb.e2.y, p0.z + tb.e2.z), box, u, 0.1f * margin, a,
+                                   e)) {
                     lo = fminf(lo, a);
                     hi = fmaxf(hi, e);
                 }
@@ -346,25 +357,31 @@ __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const 
     }
 }
 
-template <typename T>
-struct Temp {
-    T* p = nullptr;
-    ~Temp() {
+// One device allocation cut into arrays: allocating and freeing cost more
+// than the map's kernels on small geometries.
+struct Block {
+    unsigned char* p = nullptr;
+    size_t used = 0;
+    ~Block() {
         if (p) cudaFree(p);
     }
-    bool alloc(uint64_t n) {
-        if (p) cudaFree(p);
-        p = nullptr;
-        if (cudaMalloc(&p, std::max<uint64_t>(n, 1) * sizeof(T)) != cudaSuccess) {
+    // Reserves n elements; their address is valid after alloc.
+    template <typename T>
+    size_t reserve(uint64_t n) {
+        const size_t at = used;
+        used += (std::max<uint64_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+        return at;
+    }
+    bool alloc() {
+        if (cudaMalloc(&p, used) != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
         }
         return p != nullptr;
     }
-    T* release() {
-        T* r = p;
-        p = nullptr;
-        return r;
+    template <typename T>
+    T* at(size_t offset) const {
+        return reinterpret_cast<T*>(p + offset);
     }
 };
 
@@ -395,10 +412,6 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
     // triangle's edge on the exact path (0.05 nm: contact holes, whose
     // electrons hug the interfaces, 28.9 instead of 26.8 ms).
     const float margin = 0.02f + 4e-6f * scale;
-    Temp<unsigned long long> totals;
-    Temp<int32_t> big;
-    Temp<uint32_t> n_big;
-    if (!totals.alloc(4) || !big.alloc(uint64_t(n_tri)) || !n_big.alloc(1)) return false;
     const int blocks = sms * 8;
     float fine = kFineCell, reach = kReach;
     for (int tries = 0; tries < 24; ++tries, fine *= 2.0f, reach *= 2.0f) {
@@ -417,46 +430,53 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         g.ny = int(dims[1]);
         g.nz = int(dims[2]);
         const uint64_t cells = uint64_t(g.nx) * g.ny * g.nz;
-        Temp<uint32_t> count;
-        if (!count.alloc(cells)) return false;
+        // counting pass: the first words and the counts start at zero
+        Block first;
+        const size_t at_totals = first.reserve<unsigned long long>(4), at_n_big = first.reserve<uint32_t>(1),
+                     at_count = first.reserve<uint32_t>(cells), zeroed = first.used,
+                     at_big = first.reserve<int32_t>(uint64_t(n_tri));
+        if (!first.alloc() || cudaMemsetAsync(first.p, 0, zeroed, s) != cudaSuccess) return false;
+        unsigned long long* const totals = first.at<unsigned long long>(at_totals);
+        uint32_t *const n_big = first.at<uint32_t>(at_n_big), *const count = first.at<uint32_t>(at_count);
+        int32_t* const big = first.at<int32_t>(at_big);
         Lists l{};
-        l.count = count.p;
-        if (cudaMemsetAsync(count.p, 0, 4 * cells, s) != cudaSuccess || cudaMemsetAsync(n_big.p, 0, 4, s) != cudaSuccess ||
-            cudaMemsetAsync(totals.p, 0, 32, s) != cudaSuccess)
-            return false;
-        small_kernel<false><<<blocks, 256, 0, s>>>(tri, n_tri, g, l, big.p, n_big.p);
-        big_kernel<false><<<blocks, 256, 0, s>>>(tri, g, l, big.p, n_big.p);
-        total_kernel<<<blocks, 256, 0, s>>>(count.p, cells, totals.p);
+        l.count = count;
+        small_kernel<false><<<blocks, 256, 0, s>>>(tri, n_tri, g, l, big, n_big);
+        big_kernel<false><<<blocks, 256, 0, s>>>(tri, g, l, big, n_big);
+        total_kernel<<<blocks, 256, 0, s>>>(count, cells, totals);
         unsigned long long used[2] = {0, 0};
         if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpyAsync(used, totals.p, 16, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaMemcpyAsync(used, totals, 16, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess)
             return false;
         if (used[0] * kBrickCells * kRecordBytes > budget || used[1] * 4 > budget) continue;
-        Temp<int32_t> top, entry;
-        Temp<float4> rec;
-        Temp<uint64_t> start;
-        Temp<uint32_t> brick_cell, cursor;
-        if (!top.alloc(cells) || !entry.alloc(used[1]) || !rec.alloc(used[0] * kBrickCells * 2) || !start.alloc(used[0]) ||
-            !brick_cell.alloc(used[0]) || !cursor.alloc(used[0]) ||
-            cudaMemsetAsync(cursor.p, 0, 4 * std::max<uint64_t>(used[0], 1), s) != cudaSuccess)
-            return false;
-        assign_kernel<<<blocks, 256, 0, s>>>(count.p, g, totals.p + 2, top.p, start.p, brick_cell.p);
-        l.top = top.p;
-        l.start = start.p;
-        l.cursor = cursor.p;
-        l.entry = entry.p;
-        small_kernel<true><<<blocks, 256, 0, s>>>(tri, n_tri, g, l, big.p, n_big.p);
-        big_kernel<true><<<blocks, 256, 0, s>>>(tri, g, l, big.p, n_big.p);
+        Block lists, map;
+        const size_t at_entry = lists.reserve<int32_t>(used[1]), at_start = lists.reserve<uint64_t>(used[0]),
+                     at_cell = lists.reserve<uint32_t>(used[0]), at_cursor = lists.reserve<uint32_t>(used[0]);
+        const size_t at_rec = map.reserve<float4>(std::max<uint64_t>(used[0], 1) * kBrickCells * 2),
+                     at_top = map.reserve<int32_t>(cells);
+        if (!lists.alloc() || !map.alloc()) return false;
+        uint32_t *const brick_cell = lists.at<uint32_t>(at_cell), *const cursor = lists.at<uint32_t>(at_cursor);
+        uint64_t* const start = lists.at<uint64_t>(at_start);
+        int32_t* const top = map.at<int32_t>(at_top);
+        float4* const rec = map.at<float4>(at_rec);
+        if (cudaMemsetAsync(cursor, 0, 4 * std::max<uint64_t>(used[0], 1), s) != cudaSuccess) return false;
+        assign_kernel<<<blocks, 256, 0, s>>>(count, g, totals + 2, top, start, brick_cell);
+        l.top = top;
+        l.start = start;
+        l.cursor = cursor;
+        l.entry = lists.at<int32_t>(at_entry);
+        small_kernel<true><<<blocks, 256, 0, s>>>(tri, n_tri, g, l, big, n_big);
+        big_kernel<true><<<blocks, 256, 0, s>>>(tri, g, l, big, n_big);
         if (used[0])
-            record_kernel<<<unsigned(used[0]), unsigned(kBrickCells), 0, s>>>(tri, g, brick_cell.p, start.p, cursor.p,
-                                                                              entry.p, margin, rec.p);
+            record_kernel<<<unsigned(used[0]), unsigned(kBrickCells), 0, s>>>(tri, g, brick_cell, start, cursor, l.entry,
+                                                                              margin, rec);
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return false;
-        out->top = top.release();
-        out->rec = rec.release();
+        out->memory = map.p;
+        map.p = nullptr;
         dev::Clearance& m = out->map;
-        m.top = out->top;
-        m.rec = out->rec;
+        m.top = top;
+        m.rec = rec;
         m.offx = float(-double(g.lox) / fine - 0.5);
         m.offy = float(-double(g.loy) / fine - 0.5);
         m.offz = float(-double(g.loz) / fine - 0.5);
@@ -475,8 +495,7 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
 }
 
 void free_clearance(ClearanceMap* m) {
-    if (m->top) cudaFree(m->top);
-    if (m->rec) cudaFree(m->rec);
+    if (m->memory) cudaFree(m->memory);
     *m = ClearanceMap{};
 }
 

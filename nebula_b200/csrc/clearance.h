@@ -11,8 +11,7 @@ namespace nbx {
 
 struct ClearanceMap {
     dev::Clearance map{};   // what the kernels take; map.top == nullptr: no map
-    int* top = nullptr;     // device buffers behind it
-    float4* rec = nullptr;
+    void* memory = nullptr;   // the device allocation behind it
 };
 
 // Builds the map of `n_tri` triangles (three float4 each, device memory) over
