@@ -982,8 +982,15 @@ int nbx_run(nbx_ctx* ctx) {
         // entries stay on one SM); the secondary generations, written in
         // arbitrary order, from one shared cursor.
         if (!ctx->cfg.shared_pop) {
-            ctx->range_cursor.ensure(uint64_t(ctx->sms));
-            a.n_ranges = uint32_t(ctx->sms);
+            // Up to eight ranges an SM, of at least 64 primaries: an SM over
+            // denser material then has lighter parts of the scan too (contact
+            // holes, 81,920 primaries: 8.5 ms with one range an SM, 5.8 so).
+            const uint64_t parts = std::clamp<uint64_t>(ctx->n_queued / (uint64_t(ctx->sms) * 64), 1, 8);
+            a.range_sms = uint32_t(ctx->sms);
+            a.n_ranges = uint32_t(ctx->sms * parts);
+            a.range_size = uint32_t(ctx->n_queued / a.n_ranges);
+            a.range_rem = uint32_t(ctx->n_queued % a.n_ranges);
+            ctx->range_cursor.ensure(a.n_ranges);
         }
 
         // Nothing before the first launch waits on the host or on a copy

@@ -332,9 +332,17 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
     // Primaries: this SM's range of the queue first, then the following ones
     // (`probe` ranges found used up).
     uint32_t probe = 0, taken = 0;
+    // the range that a warp of this SM takes from after `p` others
+    auto range_at = [&](uint32_t p) {
+        uint32_t smid;
+        asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+        const uint32_t parts = a.n_ranges / a.range_sms;
+        return (smid + p / parts) % a.range_sms + p % parts * a.range_sms;
+    };
+    uint32_t range = a.range_cursor ? range_at(0) : 0u;
     int warps_log2 = 0;   // warps that share a cursor
     {
-        const uint32_t w = gridDim.x * (blockDim.x >> 5) / (a.range_cursor ? a.n_ranges : 1u);
+        const uint32_t w = gridDim.x * (blockDim.x >> 5) / (a.range_cursor ? a.range_sms : 1u);
         while ((1u << warps_log2) < w) ++warps_log2;
     }
     unsigned long long mine = 0;   // this lane's counter (kCnt* = lane)
@@ -514,27 +522,33 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
                     // not taken yet another one can take: with all open lanes'
                     // worth at once, a contact-hole scan whose plugs scatter
                     // more than its film ended at 22.8 ms instead of 16.5.
-                    uint32_t lo = 0, len = n_in;
+                    uint32_t lo = 0, len = n_in, got = 0, base = 0;
                     uint32_t* cursor = a.head;
                     if (a.range_cursor) {
-                        uint32_t smid;
-                        asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-                        uint32_t v = smid % a.n_ranges + probe;
-                        if (v >= a.n_ranges) v -= a.n_ranges;
-                        lo = uint32_t(uint64_t(n_in) * v / a.n_ranges);
-                        len = uint32_t(uint64_t(n_in) * (v + 1) / a.n_ranges) - lo;
-                        cursor = a.range_cursor + v;
+                        if (probe) {
+                            // past the SM's first range: `head` counts the
+                            // primaries handed out, so that the end needs no
+                            // look at every range
+                            if (lane == 0) base = *reinterpret_cast<volatile uint32_t*>(a.head);
+                            drained = __shfl_sync(kFull, base, 0) >= n_in;
+                        }
+                        lo = range * a.range_size + min(range, a.range_rem);
+                        len = a.range_size + (range < a.range_rem ? 1u : 0u);
+                        cursor = a.range_cursor + range;
                     }
-                    const uint32_t ask = min(min(uint32_t(open), kAsk), max(1u, (len - min(taken, len)) >> warps_log2));
-                    uint32_t base = 0;
-                    if (lane == 0) base = atomicAdd(cursor, ask);
-                    base = __shfl_sync(kFull, base, 0);
-                    const uint32_t got = base < len ? min(ask, len - base) : 0u;
-                    taken = base + got;
-                    if (got < ask) {
-                        taken = 0;
-                        ++probe;
-                        drained = !a.range_cursor || probe >= a.n_ranges;
+                    if (!drained) {
+                        const uint32_t ask = min(min(uint32_t(open), kAsk), max(1u, (len - min(taken, len)) >> warps_log2));
+                        if (lane == 0) base = atomicAdd(cursor, ask);
+                        base = __shfl_sync(kFull, base, 0);
+                        got = base < len ? min(ask, len - base) : 0u;
+                        taken = base + got;
+                        if (got < ask) {
+                            taken = 0;
+                            ++probe;
+                            drained = !a.range_cursor || probe >= a.n_ranges;
+                            if (!drained) range = range_at(probe);
+                        }
+                        if (a.range_cursor && got && lane == 0) atomicAdd(a.head, got);
                     }
                     const int r = rank - n1 - n2;
                     bool ended = false;
