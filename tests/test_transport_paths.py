@@ -109,12 +109,14 @@ def soup_in_a_block(seed=4):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("model", ["kieft", "penn"])
-@pytest.mark.parametrize("name", ["cube", "grating_small", "rough", "holes", "soup"])
+@pytest.mark.parametrize("name", ["cube", "grating_small", "rough", "holes", "soup", "vast"])
 def test_run_equals_single_steps(name, model, inputs):
     import nebula_b200 as nb
     from nebula_b200 import generators as g
-    tris = soup_in_a_block() if name == "soup" else inputs[name]
-    top = {"cube": 1.0, "grating_small": 75.0, "rough": 20.0, "holes": 10.0, "soup": 1.0}[name]
+    # "vast": a domain whose clearance map needs cells above the usual size
+    tris = (soup_in_a_block() if name == "soup" else
+            g.cube_geometry(size=(60000.0, 60000.0, 30000.0)) if name == "vast" else inputs[name])
+    top = {"cube": 1.0, "grating_small": 75.0, "rough": 20.0, "holes": 10.0, "soup": 1.0, "vast": 1.0}[name]
     recs = g.scan_beam(9, 9, 12, 500.0, spacing=8.0, origin=(-36.0, -36.0), z_start=top, seed=23,
                        energies=[120.0, 500.0, 2000.0])
     prim = np.concatenate([recs["pos"], recs["dir"], recs["E"][:, None]], 1).astype(np.float32)
@@ -159,3 +161,41 @@ def test_table_indices_at_the_edges(inputs):
             want = [f(C.byref(t), float(v), float(w)) for v, w in zip(x, y)]
         assert np.array_equal(got, np.array(want, np.float32), equal_nan=True), name
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["plain", "weighted", "network"])
+def test_launch_shapes_and_shallow_stacks_change_nothing(mode, inputs):
+    """The same per-primary tallies whatever the launch shape, with stacks of
+    one electron per thread (secondaries then go through the next generations'
+    queues, in learned mode with their weights) and with queues that fill whole
+    ranges, one primary and none."""
+    import nebula_b200 as nb
+    from nebula_b200 import generators as g
+    recs = g.scan_beam(16, 12, 11, 2000.0, spacing=4.0, origin=(-32.0, -24.0), seed=9)
+    want = None
+    for variant, block, depth in ((3, 256, 16), (3, 256, 1), (2, 32, 1), (4, 128, 2), (7, 128, 1), (4, 256, 64)):
+        ctx = nb.setup(inputs["grating_small"], [inputs["si"]], device=0, seed=5)
+        ctx.set_tag_range(len(recs))
+        if mode != "plain":
+            ctx.build_surface_map([-150, -150, -60], [150, 150, 60], 2.0, 20.0)
+            ctx.mlp_set_params(nb.mlp_init_params(3))
+            ctx.set_mode("learned", rr_threshold=0.6, split_threshold=0.65, max_roulette_exp=3)
+            if mode == "weighted":
+                ctx.set_importance_table(16, 16, 8)
+        ctx.set_tuning(variant, block, depth, 2)
+        got = []
+        for n in (len(recs), 1, 0, 149):
+            ctx.reset_tallies()
+            ctx.set_uid_base(0)
+            ctx.push_records(recs[:n])
+            ctx.run()
+            s = ctx.stats()
+            got += [ctx.tag_counts(0, len(recs)), ctx.tag_weights(0, len(recs)),
+                    [s[k] for k in ("steps", "events_elastic", "events_inelastic", "events_boundary", "secondaries",
+                                    "terminated", "detected", "primaries_done", "queue_overflow")]]
+        ctx.close()
+        want = want or got
+        for a, b in zip(got, want):
+            assert all(np.array_equal(x, y) for x, y in zip(a, b)), (variant, block, depth)
+    assert want[0][0].sum() > 100 and want[2][-1] == 0
