@@ -37,8 +37,11 @@ struct TrainSmem {
     Weights w;
     bf16 w2t[kHidden * kHidden];   // [in][out]
     bf16 w3t[kHidden * 16];        // [in][out padded to 16]
-    float gacc[kParams];
-    float loss;
+    // each warp's gradient of its 32 samples: every element is stored once, so
+    // no shared-memory atomics (a compare-and-swap loop for floats; B200,
+    // fitting 200,003 records twice in batches of 8,192: 4.79 -> 3.96 ms)
+    float gacc[kWarps][kParams];
+    float loss[kWarps];
     WarpBuf warp[kWarps];
 };
 
@@ -83,7 +86,7 @@ __device__ __forceinline__ float silu_grad(float z) {
 
 // Column sums of a [32][8 NT] fragment set over the warp's 32 rows.
 template <int NT>
-__device__ __forceinline__ void add_column_sums(float (*acc)[NT][4], float* dst, int n_valid_cols) {
+__device__ __forceinline__ void store_column_sums(float (*acc)[NT][4], float* dst, int n_valid_cols) {
     const int t = threadIdx.x & 3;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
@@ -94,7 +97,7 @@ __device__ __forceinline__ void add_column_sums(float (*acc)[NT][4], float* dst,
             s += __shfl_xor_sync(0xffffffffu, s, 8);
             s += __shfl_xor_sync(0xffffffffu, s, 16);
             const int col = nt * 8 + 2 * t + j;
-            if ((threadIdx.x & 31) < 4 && col < n_valid_cols) atomicAdd(dst + col, s);
+            if ((threadIdx.x & 31) < 4 && col < n_valid_cols) dst[col] = s;
         }
     }
 }
@@ -128,8 +131,8 @@ __device__ __forceinline__ void load_train_weights(TrainSmem& sm, const float* p
         const int in = i / 16, out = i % 16;
         sm.w3t[i] = __float2bfloat16_rn(out < kOut ? params[kOffW3 + out * kHidden + in] : 0.0f);
     }
-    for (int i = threadIdx.x; i < kParams; i += blockDim.x) sm.gacc[i] = 0.0f;
-    if (threadIdx.x == 0) sm.loss = 0.0f;
+    for (int i = threadIdx.x; i < kWarps * kParams; i += blockDim.x) (&sm.gacc[0][0])[i] = 0.0f;
+    if (threadIdx.x < kWarps) sm.loss[threadIdx.x] = 0.0f;
 }
 
 // One block: kWarps x 32 samples of the batch [first, first + count).
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(kWarps * 32) train_kernel(const float* params,
     __syncthreads();
     const int warp = threadIdx.x >> 5;
     WarpBuf& wb = sm.warp[warp];
+    float* const gacc = sm.gacc[warp];
     const uint64_t tile = (uint64_t(blockIdx.x) * kWarps + warp) * 32;
     const uint64_t end = first + count;
     if (first + tile < end) {
@@ -225,8 +229,8 @@ __global__ void __launch_bounds__(kWarps * 32) train_kernel(const float* params,
             db3 += __shfl_xor_sync(0xffffffffu, db3, o);
         }
         if (lane == 0) {
-            atomicAdd(&sm.loss, lsum);
-            atomicAdd(&sm.gacc[kOffB3], db3);
+            sm.loss[warp] = lsum;
+            gacc[kOffB3] = db3;
         }
         wb.d3[lane * 16] = __float2bfloat16_rn(dz);
         wb.d3t[lane] = __float2bfloat16_rn(dz);
@@ -242,7 +246,7 @@ __global__ void __launch_bounds__(kWarps * 32) train_kernel(const float* params,
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int r = frag_row(0, e), c = frag_col(nt, e);
-                    if (r < kOut) atomicAdd(&sm.gacc[kOffW3 + r * kHidden + c], g3[0][nt][e]);
+                    if (r < kOut) gacc[kOffW3 + r * kHidden + c] = g3[0][nt][e];
                 }
         }
         // dh2 = dz3 W3 ; dz2 = dh2 * silu'(z2)
@@ -261,7 +265,7 @@ __global__ void __launch_bounds__(kWarps * 32) train_kernel(const float* params,
                     wb.d2[r * kHidden + c] = db;
                     wb.d2t[c * 32 + r] = db;
                 }
-        add_column_sums<8>(acc, sm.gacc + kOffB2, kHidden);
+        store_column_sums<8>(acc, gacc + kOffB2, kHidden);
         __syncwarp();
         // dW2 = dz2^T h1
         {
@@ -274,7 +278,7 @@ __global__ void __launch_bounds__(kWarps * 32) train_kernel(const float* params,
                 for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
                     for (int e = 0; e < 4; ++e)
-                        atomicAdd(&sm.gacc[kOffW2 + frag_row(mt, e) * kHidden + frag_col(nt, e)], g2[mt][nt][e]);
+                        gacc[kOffW2 + frag_row(mt, e) * kHidden + frag_col(nt, e)] = g2[mt][nt][e];
         }
         // dh1 = dz2 W2 ; dz1 = dh1 * silu'(z1)
         zero<2, 8>(acc);
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(kWarps * 32) train_kernel(const float* params,
                     acc[mt][nt][e] = d;
                     wb.d1t[c * 32 + r] = __float2bfloat16_rn(d);
                 }
-        add_column_sums<8>(acc, sm.gacc + kOffB1, kHidden);
+        store_column_sums<8>(acc, gacc + kOffB1, kHidden);
         __syncwarp();
         // dW1 = dz1^T x
         {
@@ -304,14 +308,17 @@ __global__ void __launch_bounds__(kWarps * 32) train_kernel(const float* params,
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const int c = frag_col(nt, e);
-                        if (c < kFeatures) atomicAdd(&sm.gacc[kOffW1 + frag_row(mt, e) * kIn + c], g1[mt][nt][e]);
+                        if (c < kFeatures) gacc[kOffW1 + frag_row(mt, e) * kIn + c] = g1[mt][nt][e];
                     }
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kParams; i += blockDim.x)
-        if (sm.gacc[i] != 0.0f) atomicAdd(grad + i, sm.gacc[i]);
-    if (threadIdx.x == 0 && loss) atomicAdd(loss, sm.loss);
+    static_assert(kWarps == 2, "two warps' gradients are added here");
+    for (int i = threadIdx.x; i < kParams; i += blockDim.x) {
+        const float g = sm.gacc[0][i] + sm.gacc[1][i];
+        if (g != 0.0f) atomicAdd(grad + i, g);
+    }
+    if (threadIdx.x == 0 && loss) atomicAdd(loss, sm.loss[0] + sm.loss[1]);
 }
 
 __global__ void adam_kernel(float* params, const float* grad, float* m, float* v, float lr, float beta1, float beta2,
