@@ -754,8 +754,12 @@ def main():
     line = None
     if rank == 0:
         peak, peak_kind = measured_peaks()
-        b_event, b_parts = algorithmic_bytes_per_event(tris, mats, recs, 0x78C7E39B, penn=args.inelastic == "penn")
-        achieved = events * b_event / (sum(dev_ms) / 1000.0) / 1e9
+        # (the count needs the reference's own build; without it the figure is null)
+        import oracle
+        b_event, b_parts, achieved = None, None, None
+        if oracle.have_ref(args.inelastic == "penn"):
+            b_event, b_parts = algorithmic_bytes_per_event(tris, mats, recs, 0x78C7E39B, penn=args.inelastic == "penn")
+            achieved = events * b_event / (sum(dev_ms) / 1000.0) / 1e9
         # DRAM bytes per launch: the ncu capture's bytes per event (Kieft
         # model, this workload) times the events of one step, whose first
         # generation's launch carries the whole scan
@@ -801,8 +805,8 @@ def main():
             # is the DRAM traffic actually measured), and the kernel is bound
             # by instruction issue under warp divergence (ncu figures).
             "roofline": {"bound": "issue/L1-L2 latency", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": traffic, "dram_frac": dram_frac, "ncu": ncu,
-                         "peak_kind": peak_kind, "bytes_per_event": round(b_event, 2), "bytes_breakdown": b_parts,
+                         "frac": achieved / peak if achieved else None, "traffic": traffic, "dram_frac": dram_frac, "ncu": ncu,
+                         "peak_kind": peak_kind, "bytes_per_event": round(b_event, 2) if b_event else None, "bytes_breakdown": b_parts,
                          "kernel": "transport_kernel"},
             "clocks": clocks,
             "cpu_baseline": cpu,

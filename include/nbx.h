@@ -187,8 +187,9 @@ typedef struct {
     int32_t record_deposits;   /* keep energy-deposit records (plain mode; cpu_energydep.cpp) */
     uint64_t deposit_capacity; /* deposit records held on the device; 0 = 2^27 (3.2 GB) */
     int32_t shared_pop;        /* 0: the transport blocks on each SM pop the primaries of that SM's
-                                  contiguous range of the queue first (neighbouring primaries share
-                                  the SM's caches; push them in scan order); 1: one shared cursor */
+                                  contiguous ranges of the queue (up to eight, spread over it) first
+                                  (neighbouring primaries share the SM's caches; push them in scan
+                                  order); 1: one shared cursor */
 } nbx_config;
 
 /* One energy deposit (drivers/cpu/energydeposit_cpu_driver.h:74-96,
@@ -330,7 +331,8 @@ typedef struct {
     int32_t stack_depth;     /* parked electrons per thread (1..64, default 16), shared by the 32 threads of
                                 a warp: a secondary born with its warp's stack full goes to the next
                                 generation's queue (sample mode: each thread its own stack) */
-    int32_t chunk;           /* generation launches queued between two host reads (1..64, default 8) */
+    int32_t chunk;           /* generation launches queued between two host reads (1..64, default 8);
+                                the first generation is read back by itself */
     uint64_t queue_capacity; /* out: entries of each overflow queue in the last run */
     double sample_ms;        /* out (nbx_autotune): the sample's device time with these settings */
 } nbx_tuning;
