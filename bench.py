@@ -252,14 +252,14 @@ def measured_peaks():
 
 
 def algorithmic_bytes_per_event(tris, mat_paths, recs, seed, penn=False):
-    """Section-8(d) algorithmic bytes per event, counted by the instrumented
+    """Algorithmic bytes per event, counted by the instrumented
     CPU restatement on a fixed sample of the workload.  An inelastic event
     reads a 2-D ICDF (16 B) and a rounddown value (4 B) under Kieft, and the
     2-D ICDF, a trilinear 3-D q lookup (32 B) and a 3-D rounddown (4 B) under
     full Penn."""
     import oracle
     pg = oracle.PortGeometry(tris)
-    rms = [oracle.RefMaterial(p, penn=penn) for p in mat_paths]
+    rms = [oracle.material(p, penn=penn) for p in mat_paths]
     pms, arr = oracle.port_materials(rms)
     sample = strided_sample(recs, 2000)
     prim = np.zeros((len(sample), 7), np.float32)
@@ -754,12 +754,8 @@ def main():
     line = None
     if rank == 0:
         peak, peak_kind = measured_peaks()
-        # (the count needs the reference's own build; without it the figure is null)
-        import oracle
-        b_event, b_parts, achieved = None, None, None
-        if oracle.have_ref(args.inelastic == "penn"):
-            b_event, b_parts = algorithmic_bytes_per_event(tris, mats, recs, 0x78C7E39B, penn=args.inelastic == "penn")
-            achieved = events * b_event / (sum(dev_ms) / 1000.0) / 1e9
+        b_event, b_parts = algorithmic_bytes_per_event(tris, mats, recs, 0x78C7E39B, penn=args.inelastic == "penn")
+        achieved = events * b_event / (sum(dev_ms) / 1000.0) / 1e9
         # DRAM bytes per launch: the ncu capture's bytes per event (Kieft
         # model, this workload) times the events of one step, whose first
         # generation's launch carries the whole scan
@@ -805,8 +801,8 @@ def main():
             # is the DRAM traffic actually measured), and the kernel is bound
             # by instruction issue under warp divergence (ncu figures).
             "roofline": {"bound": "issue/L1-L2 latency", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak if achieved else None, "traffic": traffic, "dram_frac": dram_frac, "ncu": ncu,
-                         "peak_kind": peak_kind, "bytes_per_event": round(b_event, 2) if b_event else None, "bytes_breakdown": b_parts,
+                         "frac": achieved / peak, "traffic": traffic, "dram_frac": dram_frac, "ncu": ncu,
+                         "peak_kind": peak_kind, "bytes_per_event": round(b_event, 2), "bytes_breakdown": b_parts,
                          "kernel": "transport_kernel"},
             "clocks": clocks,
             "cpu_baseline": cpu,

@@ -70,9 +70,15 @@ def have_ref(penn=False):
     return os.path.exists(REF_PENN_SO if penn else REF_SO)
 
 
+class ReferenceMissing(RuntimeError):
+    """The reference's own build is not here (no source tree to build it from)."""
+
+
 def ref(penn=False):
     """The compiled reference: Kieft inelastic model, or with ``penn`` the
     stock full Penn model."""
+    if not have_ref(penn):
+        raise ReferenceMissing("the reference's own build is not here")
     if penn not in _ref:
         lib = C.CDLL(REF_PENN_SO if penn else REF_SO)
         lib.nbref_build_octree.restype = C.c_int
@@ -335,11 +341,48 @@ def ref_run(tri_path, pri_path, mat_paths, seed=0x78C7E39B, energy_threshold=0.0
 # ---------------------------------------------------------------------------
 # Port-side helpers (C restatement), fed with the reference's own octree and
 # material tables so it checks the product's kernels independently of the
-# product's host-side builders.
+# product's host-side builders.  Where the reference's build is missing, the
+# product's host builders feed it: the kernels are then still checked against
+# the restatement, the builders are not.
 # ---------------------------------------------------------------------------
+def library_octree(tris):
+    """As ref_build_octree, from the product's host builder."""
+    import nebula_b200 as nb
+    o = nb.HostOctree(nb.triangles_from_tri_array(tris))
+    t = o.triangles
+    return (o.octree_data, np.concatenate([t["r0"], t["e1"], t["e2"]], 1),
+            np.stack([t["mat_in"], t["mat_out"]], 1), o.center, o.halfsize)
+
+
+class LibraryMaterial:
+    """As RefMaterial (constants and tables), from the product's host loader."""
+
+    def __init__(self, path, penn=False):
+        import nebula_b200 as nb
+        self.penn = penn
+        self.m = nb.HostMaterial(path)
+        for name in ("barrier", "fermi", "band_gap", "phonon_loss", "recoil_const"):
+            setattr(self, name, float(getattr(self.m, name)))
+        self.max_energy = float(self.m.penn_max_energy if penn else self.m.max_energy)
+        self.names = {"in_imfp": "penn_imfp", "in_icdf": "penn_omega_icdf", "q": "penn_q_icdf",
+                      "ion3": "penn_ion"} if penn else {}
+
+    def table(self, which):
+        a, axes = self.m.tables[self.names.get(which, which)]
+        return a, tuple(float(v) for v in axes)
+
+    table3 = table
+
+
+def material(path, penn=False):
+    """A material for the C restatement: the reference's loader's, or without
+    the reference's build the product's."""
+    return RefMaterial(path, penn) if have_ref(penn) else LibraryMaterial(path, penn)
+
+
 class PortGeometry:
     def __init__(self, tris):
-        od, geom, mats, c, h = ref_build_octree(tris)
+        od, geom, mats, c, h = ref_build_octree(tris) if have_ref() else library_octree(tris)
         self.octree_data = np.ascontiguousarray(od, np.int32)
         self.tri = np.ascontiguousarray(geom, np.float32)
         self.tri_mat = np.ascontiguousarray(mats, np.int32)
@@ -363,10 +406,10 @@ class PortGeometry:
 
 
 class PortMaterial:
-    """Material for the C restatement, built from the reference loader's own
-    tables and axis parameters."""
+    """Material for the C restatement, built from the tables and axis
+    parameters of the reference's loader (or of ``material``)."""
 
-    def __init__(self, ref_mat: RefMaterial):
+    def __init__(self, ref_mat):
         self.ref = ref_mat
         self.arrays = {}
         t = {}

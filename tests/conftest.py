@@ -15,6 +15,26 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device")
 
 
+def _skip_without_reference():
+    """Tests against the reference's own build are skipped where it is missing
+    (it needs the reference's source tree)."""
+    import oracle
+    try:
+        return (yield)
+    except oracle.ReferenceMissing as e:
+        pytest.skip(str(e))
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_setup(item):
+    return (yield from _skip_without_reference())
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    return (yield from _skip_without_reference())
+
+
 @pytest.fixture(scope="session")
 def oracle_built():
     import oracle

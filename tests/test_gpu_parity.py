@@ -194,7 +194,7 @@ def test_step_vs_restatement(inputs, oracle_built):
     tris = inputs["grating"]
     ctx = nb.setup(tris, [inputs["si"]], device=0, seed=99)
     pg = oracle.PortGeometry(tris)
-    rm = oracle.RefMaterial(inputs["si"])
+    rm = oracle.material(inputs["si"])
     pms, arr = oracle.port_materials([rm])
     prm = oracle.Params(99, 0.0, rm.max_energy)
     rng = np.random.default_rng(11)
@@ -399,7 +399,7 @@ def test_whole_run_vs_restatement_same_streams(inputs, oracle_built):
     ctx = nb.setup(tris, [inputs["si"]], device=0, seed=77)
     s, se, bse = _run_gpu(ctx, recs)
     pg = oracle.PortGeometry(tris)
-    rm = oracle.RefMaterial(inputs["si"])
+    rm = oracle.material(inputs["si"])
     pms, arr = oracle.port_materials([rm])
     prim = np.zeros((len(recs), 7), np.float32)
     prim[:, 0:3] = recs["pos"]

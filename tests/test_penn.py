@@ -73,11 +73,10 @@ def test_penn_step_vs_restatement(inputs, oracle_built):
     """One step per electron on the GPU and in the C restatement (stock
     tables, same Philox uniforms): vacuum steps bit-exact, material steps
     within 1e-4 for at least 99.9 %."""
-    _need_penn_ref()
     tris = inputs["grating"]
     ctx = nb.setup(tris, [inputs["si"]], device=0, seed=41, inelastic="penn")
     pg = oracle.PortGeometry(tris)
-    rm = oracle.RefMaterial(inputs["si"], penn=True)
+    rm = oracle.material(inputs["si"], penn=True)
     pms, arr = oracle.port_materials([rm])
     prm = oracle.Params(41, 0.0, rm.max_energy, 1)
     rng = np.random.default_rng(12)

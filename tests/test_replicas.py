@@ -39,7 +39,7 @@ class OracleCtx:
     def __init__(self, tris, mat_path, seed):
         import oracle
         self.pg = oracle.PortGeometry(tris)
-        self.rm = oracle.RefMaterial(mat_path)
+        self.rm = oracle.material(mat_path)
         self.pms, self.arr = oracle.port_materials([self.rm])
         self.seed = seed
         self.uid_next = 0
