@@ -18,6 +18,23 @@
 // no triangle.  Surfaces are locally flat, so a slab is thin (only the
 // margin, on flat faces); the second one serves edges and corners.
 //
+// The margin covers the rounding of the exact test, because "meets no
+// triangle" has to mean that intersect_ray reports no hit.  With u = 2^-24,
+// |s| the distance from the triangle's corner to the ray's start and k =
+// |e1||e2| / |e1 x e2|, the test's three numerators are off by at most
+// 12 u |s| times the edges in them and its determinant by 8 u |e1||e2|, so the
+// point that it reports lies within 44 u k |s| / cos of the triangle, cos being
+// that of the ray's angle to the triangle's normal, and along that normal
+// within 12 u k |s|.  A triangle's `slack` is 24 u k |s| plus the 2.4e-6 of its
+// edges by which the test enlarges it; at an angle phi to its slab it widens
+// the slab by slack / 2 + 10 slack sin(phi), which covers rays down to a cosine
+// of 0.18 at the bound and of 0.02 at the errors that occur (a tenth of it),
+// and it is a candidate of the cells within 10 slack.  Triangles of sound
+// meshes mostly have a slack below 0.01 nm, and the margin decides; strips of
+// 1000 nm x 0.3 nm (5 nm) make the cells round them walk.  With one margin for
+// all shapes, runs through sheets of strips had 4 of 35,305 crossings fewer
+// than the walk reports (4000 nm x 4 nm) and 247 of 28,966 (8000 nm x 1 nm).
+//
 // h = 4 nm and reach = 3 nm: 99 % of the free paths are below 3 nm.  Share of
 // steps answered on 8,000-step samples (grating, rough slab, contact holes):
 // 0.92 / 0.91 / 0.83 with two slabs, 0.84 / 0.91 / 0.68 with one; h = 2 adds
@@ -47,12 +64,17 @@ struct Grid {
 
 struct TriBox {
     float3 a, e1, e2, lo, hi;
+    float3 u;      // unit normal (zero without an area)
+    float slack;   // rounding of the exact test (nm; infinite without an area)
+    float grow;    // boxes within this distance (nm) count as near
 };
 
 __device__ __forceinline__ float min3(float a, float b, float c) { return fminf(a, fminf(b, c)); }
 __device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(a, fmaxf(b, c)); }
 
-__device__ __forceinline__ TriBox load_tri(const float4* tri, int t) {
+// The normal is formed in double precision: that of a needle would be lost in
+// single precision, and with it the plane test of near_box.
+__device__ __forceinline__ TriBox load_tri(const float4* tri, int t, const Grid& g) {
     const float4 A = __ldg(tri + 3 * size_t(t)), B = __ldg(tri + 3 * size_t(t) + 1), C = __ldg(tri + 3 * size_t(t) + 2);
     TriBox r;
     r.a = make_float3(A.x, A.y, A.z);
@@ -60,20 +82,31 @@ __device__ __forceinline__ TriBox load_tri(const float4* tri, int t) {
     r.e2 = make_float3(C.x, C.y, C.z);
     r.lo = make_float3(A.x + min3(0.0f, B.x, C.x), A.y + min3(0.0f, B.y, C.y), A.z + min3(0.0f, B.z, C.z));
     r.hi = make_float3(A.x + max3(0.0f, B.x, C.x), A.y + max3(0.0f, B.y, C.y), A.z + max3(0.0f, B.z, C.z));
+    const double nx = double(B.y) * C.z - double(B.z) * C.y, ny = double(B.z) * C.x - double(B.x) * C.z,
+                 nz = double(B.x) * C.y - double(B.y) * C.x;
+    const double l2 = nx * nx + ny * ny + nz * nz;
+    const double s = l2 > 0.0 ? rsqrt(l2) : 0.0;
+    r.u = make_float3(float(nx * s), float(ny * s), float(nz * s));
+    const float b2 = B.x * B.x + B.y * B.y + B.z * B.z, c2 = C.x * C.x + C.y * C.y + C.z * C.z;
+    const float k = s > 0.0 ? sqrtf(b2) * sqrtf(c2) * float(s) : INFINITY;
+    const float dx = r.hi.x - r.lo.x, dy = r.hi.y - r.lo.y, dz = r.hi.z - r.lo.z;
+    const float size = sqrtf(dx * dx + dy * dy + dz * dz);   // at least the longest edge
+    const float near = 1.75f * (g.cell / kBrick + 2.0f * g.reach);   // diagonal of a widened fine cell
+    r.slack = 24.0f * 5.9604645e-8f * k * (size + near) + 2.4e-6f * size;
+    r.grow = fminf(10.0f * r.slack, fminf(2.0f * size, 8.0f * g.cell));
     return r;
 }
 
 // Conservative triangle / box test: bounding boxes, then the triangle's
 // plane against the box.  (cx, cy, cz) is the box centre, h its half edge.
 __device__ __forceinline__ bool near_box(const TriBox& t, float cx, float cy, float cz, float h) {
+    h += t.grow;
     if (t.lo.x > cx + h || t.hi.x < cx - h || t.lo.y > cy + h || t.hi.y < cy - h || t.lo.z > cz + h || t.hi.z < cz - h)
         return false;
-    const float nx = t.e1.y * t.e2.z - t.e1.z * t.e2.y, ny = t.e1.z * t.e2.x - t.e1.x * t.e2.z,
-                nz = t.e1.x * t.e2.y - t.e1.y * t.e2.x;
-    const float d = nx * (t.a.x - cx) + ny * (t.a.y - cy) + nz * (t.a.z - cz);
-    // 1.01: rounding of d and of the normal, relative to a box of the same size
-    const float r = (fabsf(nx) + fabsf(ny) + fabsf(nz)) * h * 1.01f +
-                    1e-6f * (fabsf(nx * (t.a.x - cx)) + fabsf(ny * (t.a.y - cy)) + fabsf(nz * (t.a.z - cz)));
+    const float x = t.a.x - cx, y = t.a.y - cy, z = t.a.z - cz;
+    const float d = t.u.x * x + t.u.y * y + t.u.z * z;
+    // 1e-6, 1.0001: rounding of the normal, the difference and the two sums
+    const float r = (fabsf(t.u.x) + fabsf(t.u.y) + fabsf(t.u.z)) * h * 1.0001f + 1e-6f * (fabsf(x) + fabsf(y) + fabsf(z));
     return !(fabsf(d) > r);
 }
 
@@ -83,7 +116,7 @@ __device__ __forceinline__ int clamp_cell(float x, int n) {
 
 // The coarse cells whose widened box a triangle's bounding box meets.
 __device__ __forceinline__ bool cell_range(const Grid& g, const TriBox& t, int3& lo, int3& n) {
-    const float inv = 1.0f / g.cell, r = g.reach;
+    const float inv = 1.0f / g.cell, r = g.reach + t.grow;
     if (t.hi.x < g.lox - r || t.lo.x > g.lox + g.nx * g.cell + r || t.hi.y < g.loy - r ||
         t.lo.y > g.loy + g.ny * g.cell + r || t.hi.z < g.loz - r || t.lo.z > g.loz + g.nz * g.cell + r)
         return false;
@@ -130,7 +163,7 @@ __global__ void __launch_bounds__(256) small_kernel(const float4* tri, int n_tri
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
     for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < n_tri; t += warps) {
-        const TriBox b = load_tri(tri, t);
+        const TriBox b = load_tri(tri, t, g);
         int3 lo, n;
         if (!cell_range(g, b, lo, n)) continue;
         const long long cells = (long long)n.x * n.y * n.z;
@@ -151,7 +184,7 @@ __global__ void __launch_bounds__(256) big_kernel(const float4* tri, Grid g, Lis
     const uint32_t nb = *n_big;
     for (uint32_t k = 0; k < nb; ++k) {
         const int t = big[k];
-        const TriBox b = load_tri(tri, t);
+        const TriBox b = load_tri(tri, t, g);
         int3 lo, n;
         if (!cell_range(g, b, lo, n)) continue;
         const long long cells = (long long)n.x * n.y * n.z;
@@ -256,27 +289,21 @@ __device__ bool clipped_extent(float3 p0, float3 p1, float3 p2, float h, float3 
     return true;
 }
 
-// One block of 64 threads per brick, one thread per fine cell.  The first slab
-// holds the candidates whose normals lie within 45 degrees of the nearest
-// one's, the second the others; each slab's normal is the mean of its
-// candidates' normals near that of its nearest, its extent that of its
-// candidates' clipped parts.
-__device__ __forceinline__ float3 unit_normal(const TriBox& t) {
-    const float nx = t.e1.y * t.e2.z - t.e1.z * t.e2.y, ny = t.e1.z * t.e2.x - t.e1.x * t.e2.z,
-                nz = t.e1.x * t.e2.y - t.e1.y * t.e2.x;
-    const float l2 = nx * nx + ny * ny + nz * nz;
-    const float s = l2 > 0.0f ? rsqrtf(l2) : 0.0f;
-    return make_float3(nx * s, ny * s, nz * s);
-}
 // +1 / -1: u lies within 45 degrees of n / of -n; 0: neither
 __device__ __forceinline__ float alike(float3 u, float3 n) {
     const float d = u.x * n.x + u.y * n.y + u.z * n.z;
     return d > 0.7f ? 1.0f : (d < -0.7f ? -1.0f : 0.0f);
 }
 
+// One block of 64 threads per brick, one thread per fine cell.  The first slab
+// holds the candidates whose normals lie within 45 degrees of the nearest
+// one's, the second the others; each slab's normal is the mean of its
+// candidates' normals near that of its nearest, its extent that of its
+// candidates' clipped parts, each widened by its margin.
 __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const float4* tri, Grid g, const uint32_t* brick_cell,
                                                                          const uint64_t* start, const uint32_t* n_entry,
-                                                                         const int32_t* entry, float margin, float4* rec) {
+                                                                         const int32_t* entry, float margin, float rounding,
+                                                                         float4* rec) {
     const uint32_t b = blockIdx.x;
     const uint32_t c = brick_cell[b];
     const int cx = int(c % g.nx), cy = int((c / g.nx) % g.ny), cz = int(c / (uint32_t(g.nx) * g.ny));
@@ -293,34 +320,33 @@ __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const 
         // this slab's nearest candidate
         float best = INFINITY;
         int bi = -1;
+        float3 near = make_float3(0.0f, 0.0f, 0.0f);
         for (int k = 0; k < n; ++k) {
             const int t = __ldg(list + k);
-            const TriBox tb = load_tri(tri, t);
-            if (!near_box(tb, px, py, pz, box) || (slab == 1 && alike(unit_normal(tb), first) != 0.0f)) continue;
+            const TriBox tb = load_tri(tri, t, g);
+            if (!near_box(tb, px, py, pz, box) || (slab == 1 && alike(tb.u, first) != 0.0f)) continue;
             const float d2 = dev::dist2_to_triangle(tri, t, px, py, pz);
             // (ties: the lowest index, so that the record does not depend on the list's order)
             if (d2 < best || (d2 == best && t < bi) || bi < 0) {
                 best = d2;
                 bi = t;
+                near = tb.u;
             }
         }
         float4 out = make_float4(0.0f, 0.0f, 0.0f, -2.0f);   // nothing near: n . q - c = 2 everywhere
+        // a first slab without a normal (zero area) takes every candidate
+        const bool all = slab == 0 && bi >= 0 && near.x == 0.0f && near.y == 0.0f && near.z == 0.0f;
         if (bi >= 0) {
-            float3 u = unit_normal(load_tri(tri, bi));
-            // a first slab without a normal (zero area) takes every candidate
-            const bool all = slab == 0 && u.x == 0.0f && u.y == 0.0f && u.z == 0.0f;
-            const float3 near = u;
             if (slab == 0) first = near;
             float sx = 0.0f, sy = 0.0f, sz = 0.0f;
             for (int k = 0; k < n; ++k) {
-                const TriBox tb = load_tri(tri, __ldg(list + k));
+                const TriBox tb = load_tri(tri, __ldg(list + k), g);
                 if (!near_box(tb, px, py, pz, box)) continue;
-                const float3 v = unit_normal(tb);
-                if (slab == 1 && alike(v, first) != 0.0f) continue;
-                const float s = alike(v, near);
-                sx += s * v.x;
-                sy += s * v.y;
-                sz += s * v.z;
+                if (slab == 1 && alike(tb.u, first) != 0.0f) continue;
+                const float s = alike(tb.u, near);
+                sx += s * tb.u.x;
+                sy += s * tb.u.y;
+                sz += s * tb.u.z;
             }
             float l2 = sx * sx + sy * sy + sz * sz;
             if (!(l2 > 1e-12f)) {   // no usable normal (degenerate triangles): any direction serves
@@ -328,32 +354,35 @@ __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const 
                 sz = l2 = 1.0f;
             }
             const float s = rsqrtf(l2);
-            u = make_float3(sx * s, sy * s, sz * s);
+            const float3 u = make_float3(sx * s, sy * s, sz * s);
             float lo = INFINITY, hi = -INFINITY;
             for (int k = 0; k < n; ++k) {
-                const TriBox tb = load_tri(tri, __ldg(list + k));
+                const TriBox tb = load_tri(tri, __ldg(list + k), g);
                 if (!near_box(tb, px, py, pz, box)) continue;
-                if (!all && (alike(unit_normal(tb), first) != 0.0f) != (slab == 0)) continue;
+                if (!all && (alike(tb.u, first) != 0.0f) != (slab == 0)) continue;
                 const float3 p0 = make_float3(tb.a.x - px, tb.a.y - py, tb.a.z - pz);
+                const float co = tb.u.x * u.x + tb.u.y * u.y + tb.u.z * u.z;
+                const float m = fmaxf(margin, tb.slack * (0.5f + 10.0f * sqrtf(fmaxf(1.0f - co * co, 0.0f)))) + rounding;
                 float a, e;
                 if (clipped_extent(p0, make_float3(p0.x + tb.e1.x, p0.y + tb.e1.y, p0.z + tb.e1.z),
-                                   make_float3(p0.x + tb.e2.x, p0.y + tb.e2.y, p0.z + tb.e2.z), box, u, 0.1f * margin, a,
-                                   e)) {
-                    lo = fminf(lo, a);
-                    hi = fmaxf(hi, e);
+                                   make_float3(p0.x + tb.e2.x, p0.y + tb.e2.y, p0.z + tb.e2.z), box + tb.grow, u,
+                                   0.1f * margin, a, e)) {
+                    lo = fminf(lo, a - m);
+                    hi = fmaxf(hi, e + m);
                 }
             }
-            if (hi >= lo) {
-                const float inv = 1.0f / (0.5f * (hi - lo) + margin);
+            if (hi - lo < 1e6f * g.reach) {
+                const float inv = 2.0f / (hi - lo);
                 out = make_float4(u.x * inv, u.y * inv, u.z * inv, 0.5f * (hi + lo) * inv);
-            }
-            if (all) {   // nothing is left for the second slab
-                rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i)] = out;
-                rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i) + 1] = make_float4(0.0f, 0.0f, 0.0f, -2.0f);
-                return;
+            } else if (hi >= lo) {
+                out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // no bound on a candidate's rounding: every step walks
             }
         }
         rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i) + slab] = out;
+        if (all) {   // nothing is left for the second slab
+            rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i) + 1] = make_float4(0.0f, 0.0f, 0.0f, -2.0f);
+            return;
+        }
     }
 }
 
@@ -411,13 +440,13 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
     // leaves a factor of sixty.  0.02 nm on top keeps steps that graze a
     // triangle's edge on the exact path (0.05 nm: contact holes, whose
     // electrons hug the interfaces, 28.9 instead of 26.8 ms).
-    const float margin = 0.02f + 4e-6f * scale;
+    const float margin = 0.02f, rounding = 4e-6f * scale;
     const int blocks = sms * 8;
     float fine = kFineCell, reach = kReach;
     for (int tries = 0; tries < 24; ++tries, fine *= 2.0f, reach *= 2.0f) {
         Grid g{};
         g.cell = fine * kBrick;
-        g.reach = reach + margin;
+        g.reach = reach + margin + rounding;
         g.lox = center[0] - half[0];
         g.loy = center[1] - half[1];
         g.loz = center[2] - half[2];
@@ -470,7 +499,7 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         big_kernel<true><<<blocks, 256, 0, s>>>(tri, g, l, big, n_big);
         if (used[0])
             record_kernel<<<unsigned(used[0]), unsigned(kBrickCells), 0, s>>>(tri, g, brick_cell, start, cursor, l.entry,
-                                                                              margin, rec);
+                                                                              margin, rounding, rec);
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return false;
         out->memory = map.p;
         map.p = nullptr;

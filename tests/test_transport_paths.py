@@ -132,6 +132,47 @@ def test_run_equals_single_steps(name, model, inputs):
     assert [s[k] for k in ("steps", "events_inelastic", "events_elastic", "events_boundary")] == events.tolist()
 
 
+def strip_sheets(length, width, span=70.0, n_sheets=12, gap=2.0, seed=5):
+    """Parallel sheets in a general direction, cut into strips of two
+    triangles, materials 0 and 1 in turn: where a rounded edge is extruded
+    along a line, the exact test's rounding grows with the strips' length
+    over their width and with their length."""
+    q = np.linalg.qr(np.random.default_rng(seed).normal(size=(3, 3)))[0]
+    shift = np.random.default_rng(seed).uniform(0, width, n_sheets)
+    k, half = int(span / width), 0.5 * length * q[:, 0]
+    v = []
+    for s in range(n_sheets):
+        o = np.array([0.0, 0.0, -12.0]) + q[:, 2] * gap * (s - n_sheets / 2) + q[:, 1] * shift[s]
+        for j in range(k):
+            a, b = o + q[:, 1] * (j - k / 2) * width, o + q[:, 1] * (j + 1 - k / 2) * width
+            v += [(a - half, a + half, b + half), (a - half, b + half, b - half)]
+    t = np.zeros(len(v), formats.TRI_DTYPE)
+    t["v"] = np.array(v)
+    t["mat_in"], t["mat_out"] = np.repeat(np.arange(n_sheets) % 2, 2 * k), np.repeat((np.arange(n_sheets) + 1) % 2, 2 * k)
+    return t
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length,width", [(1000.0, 0.3), (3000.0, 1.0), (8000.0, 1.0), (4000.0, 4.0)])
+def test_run_equals_single_steps_near_strips(length, width, inputs):
+    import nebula_b200 as nb
+    from nebula_b200 import generators as g
+    tris = np.concatenate([g.cube_geometry(size=(300.0, 300.0, 200.0)), strip_sheets(length, width)])
+    recs = g.scan_beam(9, 9, 12, 500.0, spacing=4.0, origin=(-18.0, -18.0), z_start=1.0, seed=23,
+                       energies=[120.0, 500.0, 2000.0])
+    prim = np.concatenate([recs["pos"], recs["dir"], recs["E"][:, None]], 1).astype(np.float32)
+    ctx = nb.setup(tris, [inputs["si"], inputs["sio2"]], device=0, seed=77)
+    ctx.push(prim, np.arange(len(prim), dtype=np.uint32))
+    ctx.run()
+    s = ctx.stats()
+    got = ctx.tag_counts(0, len(prim))
+    se, bse, events = cascades_step_by_step(ctx, prim)
+    ctx.close()
+    assert events[3] > 20000   # most of them in the strips
+    assert np.array_equal(got[0], se) and np.array_equal(got[1], bse)
+    assert [s[k] for k in ("steps", "events_inelastic", "events_elastic", "events_boundary")] == events.tolist()
+
+
 @pytest.mark.gpu
 def test_table_indices_at_the_edges(inputs):
     """Table lookups whose index is clamped: below and above the axes, on
