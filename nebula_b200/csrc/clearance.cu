@@ -62,7 +62,7 @@ struct Grid {
     float reach;           // widening of the boxes (margin included)
 };
 
-struct TriBox {
+struct alignas(16) TriBox {
     float3 a, e1, e2, lo, hi;
     float3 u;      // unit normal (zero without an area)
     float slack;   // rounding of the exact test (nm; infinite without an area)
@@ -241,52 +241,69 @@ __global__ void __launch_bounds__(256) assign_kernel(const uint32_t* count, Grid
 }
 
 // Extent along n of the part of a triangle inside the box of half edge h
-// round the origin; false when there is none.  A triangle that lies in the
-// box, or whose extent along n is next to nothing anyway (a flat face under
-// its own normal), counts whole; the others are clipped (Sutherland-Hodgman,
-// in local memory: on a flat geometry it was most of the map's time).
-__device__ bool clipped_extent(float3 p0, float3 p1, float3 p2, float h, float3 n, float flat, float& lo, float& hi) {
-    const float d0 = n.x * p0.x + n.y * p0.y + n.z * p0.z, d1 = n.x * p1.x + n.y * p1.y + n.z * p1.z,
-                d2 = n.x * p2.x + n.y * p2.y + n.z * p2.z;
-    lo = min3(d0, d1, d2);
-    hi = max3(d0, d1, d2);
-    const float reach = max3(max3(fabsf(p0.x), fabsf(p0.y), fabsf(p0.z)), max3(fabsf(p1.x), fabsf(p1.y), fabsf(p1.z)),
-                             max3(fabsf(p2.x), fabsf(p2.y), fabsf(p2.z)));
-    if (reach <= h || hi - lo <= flat) return true;
-    // a convex polygon gains at most one vertex per plane (nine in all); one
-    // that rounding has folded could gain more, and keeps what it has then
-    // (clipping less only widens the extent)
-    constexpr int kMax = 20;
-    float3 v[kMax], w[kMax];
-    v[0] = p0;
-    v[1] = p1;
-    v[2] = p2;
-    int k = 3;
-    for (int side = 0; side < 6 && k <= kMax / 2; ++side) {
-        const int ax = side >> 1;
-        const float s = (side & 1) ? -1.0f : 1.0f;
-        int m = 0;
-        for (int i = 0; i < k; ++i) {
-            const float3 a = v[i], b = v[i + 1 < k ? i + 1 : 0];
-            const float da = h - s * (ax == 0 ? a.x : ax == 1 ? a.y : a.z);
-            const float db = h - s * (ax == 0 ? b.x : ax == 1 ? b.y : b.z);
-            if (da >= 0.0f) w[m++] = a;
-            if ((da >= 0.0f) != (db >= 0.0f)) {
-                const float f = da / (da - db);
-                w[m++] = make_float3(a.x + f * (b.x - a.x), a.y + f * (b.y - a.y), a.z + f * (b.z - a.z));
-            }
+// round the origin; false when there is none.  p is the triangle's corner.  A
+// triangle that lies in the box, or whose extent along n is next to nothing
+// anyway (a flat face under its own normal), counts whole.  For the others the
+// part's corners are the ends of the triangle's edges inside the box and the
+// points where the box's edges pass through the triangle.  (A corner that
+// rounding loses lies within it of one that is kept.)  No polygon is kept:
+// clipping plane by plane needs arrays in local memory, which were most of the
+// map's time.
+__device__ __forceinline__ bool clipped_extent(const TriBox& t, float3 p, float h, float3 n, float flat, float& lo, float& hi) {
+    const float3 e1 = t.e1, e2 = t.e2;
+    const float dp = n.x * p.x + n.y * p.y + n.z * p.z, d1 = n.x * e1.x + n.y * e1.y + n.z * e1.z,
+                d2 = n.x * e2.x + n.y * e2.y + n.z * e2.z;
+    lo = dp + min3(0.0f, d1, d2);
+    hi = dp + max3(0.0f, d1, d2);
+    const float far = max3(max3(fabsf(p.x), fabsf(p.y), fabsf(p.z)),
+                           max3(fabsf(p.x + e1.x), fabsf(p.y + e1.y), fabsf(p.z + e1.z)),
+                           max3(fabsf(p.x + e2.x), fabsf(p.y + e2.y), fabsf(p.z + e2.z)));
+    if (far <= h || hi - lo <= flat) return true;
+    lo = INFINITY;
+    hi = -INFINITY;
+    // the triangle's edges: from a along d, in the box for parameters [s, e]
+    auto edge = [&](float3 a, float3 d, float da, float dd) {
+        const float ix = 1.0f / d.x, iy = 1.0f / d.y, iz = 1.0f / d.z;
+        const float x0 = (-h - a.x) * ix, x1 = (h - a.x) * ix, y0 = (-h - a.y) * iy, y1 = (h - a.y) * iy,
+                    z0 = (-h - a.z) * iz, z1 = (h - a.z) * iz;
+        const float s = fmaxf(0.0f, max3(fminf(x0, x1), fminf(y0, y1), fminf(z0, z1)));
+        const float e = fminf(1.0f, min3(fmaxf(x0, x1), fmaxf(y0, y1), fmaxf(z0, z1)));
+        if (s <= e) {
+            const float u = da + dd * s, v = da + dd * e;
+            lo = min3(lo, u, v);
+            hi = max3(hi, u, v);
         }
-        k = m;
-        if (k == 0) return false;
-        for (int i = 0; i < k; ++i) v[i] = w[i];
+    };
+    edge(p, e1, dp, d1);
+    edge(p, e2, dp, d2);
+    edge(make_float3(p.x + e1.x, p.y + e1.y, p.z + e1.z), make_float3(e2.x - e1.x, e2.y - e1.y, e2.z - e1.z), dp + d1, d2 - d1);
+    // the box's edges along x, y and z: the point of the triangle's plane on
+    // each, and its barycentric coordinates times twice the area, f, g and
+    // area - f - g
+    const float3 u = t.u, f1 = make_float3(u.y * e1.z - u.z * e1.y, u.z * e1.x - u.x * e1.z, u.x * e1.y - u.y * e1.x),
+                 f2 = make_float3(u.y * e2.z - u.z * e2.y, u.z * e2.x - u.x * e2.z, u.x * e2.y - u.y * e2.x);
+    const float area = f1.x * e2.x + f1.y * e2.y + f1.z * e2.z, at = u.x * p.x + u.y * p.y + u.z * p.z;
+    const float size = fabsf(e1.x) + fabsf(e1.y) + fabsf(e1.z) + fabsf(e2.x) + fabsf(e2.y) + fabsf(e2.z);
+    const float tol = -2e-6f * size * (size + 2.0f * h);
+    auto corner = [&](float x, float y, float z) {
+        const float rx = x - p.x, ry = y - p.y, rz = z - p.z;
+        const float f = f1.x * rx + f1.y * ry + f1.z * rz, g = -(f2.x * rx + f2.y * ry + f2.z * rz);
+        if (f >= tol && g >= tol && area - f - g >= tol) {
+            const float d = n.x * x + n.y * y + n.z * z;
+            lo = fminf(lo, d);
+            hi = fmaxf(hi, d);
+        }
+    };
+    const float ux = 1.0f / u.x, uy = 1.0f / u.y, uz = 1.0f / u.z;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float a = (k & 1) ? h : -h, b = (k & 2) ? h : -h;
+        const float x = (at - u.y * a - u.z * b) * ux, y = (at - u.x * a - u.z * b) * uy, z = (at - u.x * a - u.y * b) * uz;
+        if (fabsf(x) <= h) corner(x, a, b);
+        if (fabsf(y) <= h) corner(a, y, b);
+        if (fabsf(z) <= h) corner(a, b, z);
     }
-    lo = hi = n.x * v[0].x + n.y * v[0].y + n.z * v[0].z;
-    for (int i = 1; i < k; ++i) {
-        const float d = n.x * v[i].x + n.y * v[i].y + n.z * v[i].z;
-        lo = fminf(lo, d);
-        hi = fmaxf(hi, d);
-    }
-    return true;
+    return hi >= lo;
 }
 
 // +1 / -1: u lies within 45 degrees of n / of -n; 0: neither
@@ -295,15 +312,88 @@ __device__ __forceinline__ float alike(float3 u, float3 n) {
     return d > 0.7f ? 1.0f : (d < -0.7f ? -1.0f : 0.0f);
 }
 
+// A slab of a fine cell while its record is made.
+struct Slab {
+    float best = INFINITY;   // nearest candidate: squared distance, index, normal
+    int t = -1;
+    float3 near = {0.0f, 0.0f, 0.0f};
+    float3 sum = {0.0f, 0.0f, 0.0f};   // of the normals near that one
+    float3 u = {0.0f, 0.0f, 1.0f};     // the slab's normal
+    float lo = INFINITY, hi = -INFINITY;
+
+    // (ties: the lowest index, so that the record does not depend on the list's order)
+    __device__ __forceinline__ void nearest(const TriBox& b, int i, float px, float py, float pz) {
+        float qx, qy, qz;
+        dev::closest_point_on_triangle(px, py, pz, make_float4(b.a.x, b.a.y, b.a.z, 0.0f),
+                                       make_float4(b.e1.x, b.e1.y, b.e1.z, 0.0f),
+                                       make_float4(b.e2.x, b.e2.y, b.e2.z, 0.0f), &qx, &qy, &qz);
+        const float d2 = (px - qx) * (px - qx) + (py - qy) * (py - qy) + (pz - qz) * (pz - qz);
+        if (d2 < best || (d2 == best && i < t) || t < 0) {
+            best = d2;
+            t = i;
+            near = b.u;
+        }
+    }
+    __device__ __forceinline__ void add_normal(const TriBox& b) {
+        const float s = alike(b.u, near);
+        sum.x += s * b.u.x;
+        sum.y += s * b.u.y;
+        sum.z += s * b.u.z;
+    }
+    __device__ __forceinline__ void set_normal() {
+        const float l2 = sum.x * sum.x + sum.y * sum.y + sum.z * sum.z;
+        if (!(l2 > 1e-12f)) return;   // no usable normal (degenerate triangles): any direction serves
+        const float s = rsqrtf(l2);
+        u = make_float3(sum.x * s, sum.y * s, sum.z * s);
+    }
+    __device__ __forceinline__ void extend(const TriBox& b, float px, float py, float pz, float box, float margin,
+                                           float rounding) {
+        const float3 p = make_float3(b.a.x - px, b.a.y - py, b.a.z - pz);
+        const float co = b.u.x * u.x + b.u.y * u.y + b.u.z * u.z;
+        const float m = fmaxf(margin, b.slack * (0.5f + 10.0f * sqrtf(fmaxf(1.0f - co * co, 0.0f)))) + rounding;
+        float x, y;
+        if (clipped_extent(b, p, box + b.grow, u, 0.1f * margin, x, y)) {
+            lo = fminf(lo, x - m);
+            hi = fmaxf(hi, y + m);
+        }
+    }
+    __device__ __forceinline__ float4 record(float most) const {
+        if (!(hi >= lo)) return make_float4(0.0f, 0.0f, 0.0f, -2.0f);   // nothing near: n . q - c = 2 everywhere
+        // no bound on a candidate's rounding: every step walks
+        if (!(hi - lo < most)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float inv = 2.0f / (hi - lo);
+        return make_float4(u.x * inv, u.y * inv, u.z * inv, 0.5f * (hi + lo) * inv);
+    }
+};
+
 // One block of 64 threads per brick, one thread per fine cell.  The first slab
 // holds the candidates whose normals lie within 45 degrees of the nearest
 // one's, the second the others; each slab's normal is the mean of its
 // candidates' normals near that of its nearest, its extent that of its
 // candidates' clipped parts, each widened by its margin.
+//
+// Bound by the instructions of clipped_extent and near_box (a brick of the
+// contact holes has 31 candidates, each near a third of its cells).  The block
+// keeps its candidates in shared memory, 64 at a time, and goes over them four
+// times (nearest; normal, and the second slab's nearest; extent, and the second
+// slab's normal; the second slab's extent).  B200, against every thread reading
+// and preparing every candidate six times and clipping polygons in local
+// memory: 16 x 16 contact holes (89,079 bricks, 2.8 million candidates) 16.2 ->
+// 5.6 ms, 8 x 8 holes 4.5 -> 1.6 ms; nbx_set_geometry 29.2 -> 19.5 and 9.0 ->
+// 7.8 ms, of which 11 and 3 ms are the octree and the triangles.
+//
+// A brick of more than kMaxList candidates (a mesh far finer than the cells, as
+// in a domain that is far larger) gets records under which every step walks:
+// there its slabs would fill their cells, and finding that out took 370 ms for
+// 132,108 triangles in one cell of a 1 mm domain (8 ms with the limit).
+constexpr int kMaxList = 1 << 14;
 __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const float4* tri, Grid g, const uint32_t* brick_cell,
                                                                          const uint64_t* start, const uint32_t* n_entry,
                                                                          const int32_t* entry, float margin, float rounding,
                                                                          float4* rec) {
+    constexpr int kTile = kBrick * kBrick * kBrick;
+    __shared__ TriBox tile[kTile];
+    __shared__ int tile_t[kTile];
     const uint32_t b = blockIdx.x;
     const uint32_t c = brick_cell[b];
     const int cx = int(c % g.nx), cy = int((c / g.nx) % g.ny), cz = int(c / (uint32_t(g.nx) * g.ny));
@@ -314,76 +404,55 @@ __global__ void __launch_bounds__(kBrick * kBrick * kBrick) record_kernel(const 
     const float box = 0.5f * h + g.reach;
     const int32_t* list = entry + start[b];
     const int n = int(n_entry[b]);
-    float3 first = make_float3(0.0f, 0.0f, 0.0f);   // normal that marks the first slab's candidates
-#pragma unroll 1
-    for (int slab = 0; slab < 2; ++slab) {
-        // this slab's nearest candidate
-        float best = INFINITY;
-        int bi = -1;
-        float3 near = make_float3(0.0f, 0.0f, 0.0f);
-        for (int k = 0; k < n; ++k) {
-            const int t = __ldg(list + k);
-            const TriBox tb = load_tri(tri, t, g);
-            if (!near_box(tb, px, py, pz, box) || (slab == 1 && alike(tb.u, first) != 0.0f)) continue;
-            const float d2 = dev::dist2_to_triangle(tri, t, px, py, pz);
-            // (ties: the lowest index, so that the record does not depend on the list's order)
-            if (d2 < best || (d2 == best && t < bi) || bi < 0) {
-                best = d2;
-                bi = t;
-                near = tb.u;
-            }
-        }
-        float4 out = make_float4(0.0f, 0.0f, 0.0f, -2.0f);   // nothing near: n . q - c = 2 everywhere
-        // a first slab without a normal (zero area) takes every candidate
-        const bool all = slab == 0 && bi >= 0 && near.x == 0.0f && near.y == 0.0f && near.z == 0.0f;
-        if (bi >= 0) {
-            if (slab == 0) first = near;
-            float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-            for (int k = 0; k < n; ++k) {
-                const TriBox tb = load_tri(tri, __ldg(list + k), g);
-                if (!near_box(tb, px, py, pz, box)) continue;
-                if (slab == 1 && alike(tb.u, first) != 0.0f) continue;
-                const float s = alike(tb.u, near);
-                sx += s * tb.u.x;
-                sy += s * tb.u.y;
-                sz += s * tb.u.z;
-            }
-            float l2 = sx * sx + sy * sy + sz * sz;
-            if (!(l2 > 1e-12f)) {   // no usable normal (degenerate triangles): any direction serves
-                sx = sy = 0.0f;
-                sz = l2 = 1.0f;
-            }
-            const float s = rsqrtf(l2);
-            const float3 u = make_float3(sx * s, sy * s, sz * s);
-            float lo = INFINITY, hi = -INFINITY;
-            for (int k = 0; k < n; ++k) {
-                const TriBox tb = load_tri(tri, __ldg(list + k), g);
-                if (!near_box(tb, px, py, pz, box)) continue;
-                if (!all && (alike(tb.u, first) != 0.0f) != (slab == 0)) continue;
-                const float3 p0 = make_float3(tb.a.x - px, tb.a.y - py, tb.a.z - pz);
-                const float co = tb.u.x * u.x + tb.u.y * u.y + tb.u.z * u.z;
-                const float m = fmaxf(margin, tb.slack * (0.5f + 10.0f * sqrtf(fmaxf(1.0f - co * co, 0.0f)))) + rounding;
-                float a, e;
-                if (clipped_extent(p0, make_float3(p0.x + tb.e1.x, p0.y + tb.e1.y, p0.z + tb.e1.z),
-                                   make_float3(p0.x + tb.e2.x, p0.y + tb.e2.y, p0.z + tb.e2.z), box + tb.grow, u,
-                                   0.1f * margin, a, e)) {
-                    lo = fminf(lo, a - m);
-                    hi = fmaxf(hi, e + m);
-                }
-            }
-            if (hi - lo < 1e6f * g.reach) {
-                const float inv = 2.0f / (hi - lo);
-                out = make_float4(u.x * inv, u.y * inv, u.z * inv, 0.5f * (hi + lo) * inv);
-            } else if (hi >= lo) {
-                out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // no bound on a candidate's rounding: every step walks
-            }
-        }
-        rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i) + slab] = out;
-        if (all) {   // nothing is left for the second slab
-            rec[2 * (size_t(b) * (kBrick * kBrick * kBrick) + i) + 1] = make_float4(0.0f, 0.0f, 0.0f, -2.0f);
-            return;
-        }
+    float4* const out = rec + 2 * (size_t(b) * kTile + i);
+    if (n > kMaxList) {   // (the whole block)
+        out[0] = out[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return;
     }
+    bool loaded = false;
+    // f(candidate, index) for the candidates near this thread's cell; called by the whole block
+    auto each = [&](auto&& f) {
+        for (int at = 0; at < n; at += kTile) {
+            if (!loaded || n > kTile) {
+                __syncthreads();
+                if (at + i < n) {
+                    tile_t[i] = __ldg(list + at + i);
+                    tile[i] = load_tri(tri, tile_t[i], g);
+                }
+                __syncthreads();
+                loaded = true;
+            }
+            const int m = min(kTile, n - at);
+            for (int k = 0; k < m; ++k)
+                if (near_box(tile[k], px, py, pz, box)) f(tile[k], tile_t[k]);
+        }
+    };
+    Slab s0, s1;
+    each([&](const TriBox& t, int k) { s0.nearest(t, k, px, py, pz); });
+    // (a first slab without a normal, of a triangle without an area, takes every candidate)
+    const bool all = s0.near.x == 0.0f && s0.near.y == 0.0f && s0.near.z == 0.0f;
+    auto in_first = [&](const TriBox& t) { return all || alike(t.u, s0.near) != 0.0f; };
+    each([&](const TriBox& t, int k) {
+        if (in_first(t))
+            s0.add_normal(t);
+        else
+            s1.nearest(t, k, px, py, pz);
+    });
+    s0.set_normal();
+    each([&](const TriBox& t, int) {
+        if (in_first(t))
+            s0.extend(t, px, py, pz, box, margin, rounding);
+        else
+            s1.add_normal(t);
+    });
+    if (__syncthreads_or(s1.t >= 0)) {
+        s1.set_normal();
+        each([&](const TriBox& t, int) {
+            if (!in_first(t)) s1.extend(t, px, py, pz, box, margin, rounding);
+        });
+    }
+    out[0] = s0.record(1e6f * g.reach);
+    out[1] = s1.record(1e6f * g.reach);
 }
 
 // One device allocation cut into arrays: allocating and freeing cost more
