@@ -246,6 +246,11 @@ int nbx_create(nbx_ctx** ctx, const nbx_config* cfg);
 void nbx_destroy(nbx_ctx* ctx);
 const char* nbx_last_error(nbx_ctx* ctx);
 int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* oct);
+/* The clearance map that nbx_set_geometry built (no counterpart in the
+ * reference): the edge of its fine cells in nm and its device memory.  4 nm,
+ * doubled until the map fits an eighth of the free memory (at most 4 GiB); 0
+ * and 0: no memory for one, and every step walks the octree (same results). */
+int nbx_get_clearance(nbx_ctx* ctx, float* cell, uint64_t* bytes);
 int nbx_add_material(nbx_ctx* ctx, const nbx_material* mat);
 /* Per-primary tallies are kept for tags [0, n_tags). */
 int nbx_set_tag_range(nbx_ctx* ctx, uint64_t n_tags);

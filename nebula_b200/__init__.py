@@ -135,6 +135,7 @@ def lib():
         "nbx_destroy": (None, [_vp]),
         "nbx_last_error": (C.c_char_p, [_vp]),
         "nbx_set_geometry": (C.c_int, [_vp, C.POINTER(Octree)]),
+        "nbx_get_clearance": (C.c_int, [_vp, C.POINTER(C.c_float), C.POINTER(C.c_uint64)]),
         "nbx_add_material": (C.c_int, [_vp, C.POINTER(Material)]),
         "nbx_set_tag_range": (C.c_int, [_vp, C.c_uint64]),
         "nbx_push": (C.c_int, [_vp, _vp, _vp, C.c_uint64, C.POINTER(C.c_uint64)]),
@@ -356,6 +357,12 @@ class Context:
     def set_geometry(self, octree: HostOctree):
         self._ck(self.L.nbx_set_geometry(self.h, octree._p))
         self.octree = octree
+
+    def clearance(self) -> dict:
+        """The geometry's clearance map: fine cell edge (nm) and device bytes, 0 without one."""
+        cell, n = C.c_float(), C.c_uint64()
+        self._ck(self.L.nbx_get_clearance(self.h, C.byref(cell), C.byref(n)))
+        return {"cell": cell.value, "bytes": n.value}
 
     def add_material(self, mat: HostMaterial):
         self._ck(self.L.nbx_add_material(self.h, mat._p))

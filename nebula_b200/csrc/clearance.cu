@@ -470,12 +470,13 @@ struct Block {
         used += (std::max<uint64_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
         return at;
     }
-    bool alloc() {
-        if (cudaMalloc(&p, used) != cudaSuccess) {
+    cudaError_t alloc() {
+        const cudaError_t e = cudaMalloc(&p, used);
+        if (e != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
         }
-        return p != nullptr;
+        return e;
     }
     template <typename T>
     T* at(size_t offset) const {
@@ -485,25 +486,25 @@ struct Block {
 
 }  // namespace
 
-// Cell size: kFineCell, doubled until the coarse grid and the records fit
-// their budgets (kMaxCells coarse cells; an eighth of the free memory, at
-// most kMaxRecordBytes, for the records).  The reach grows with the cells.
-bool build_clearance(const float4* tri, int n_tri, const float center[3], const float half[3], int sms, cudaStream_t s,
-                     ClearanceMap* out) {
+// Cell size: kFineCell, doubled until the map, and the lists it is made from,
+// each fit an eighth of the free memory (at most kMaxBytes) and can be
+// allocated, with at most kMaxCells coarse cells.  The reach grows with the
+// cells.
+cudaError_t build_clearance(const float4* tri, int n_tri, const float center[3], const float half[3], int sms,
+                            cudaStream_t s, ClearanceMap* out) {
     constexpr float kFineCell = 4.0f, kReach = 3.0f;
-    constexpr uint64_t kMaxCells = 1ull << 26, kMaxRecordBytes = 4ull << 30;
-    constexpr uint64_t kBrickCells = kBrick * kBrick * kBrick, kRecordBytes = 2 * sizeof(float4);
+    constexpr uint64_t kMaxCells = 1ull << 26, kMaxBytes = 4ull << 30;
+    constexpr uint64_t kBrickCells = kBrick * kBrick * kBrick;
     float scale = 0.0f;   // largest coordinate: sizes the rounding margin
     for (int i = 0; i < 3; ++i) {
-        if (!(half[i] > 0.0f) || !(half[i] < 1e18f) || !(std::fabs(center[i]) < 1e18f)) return false;
+        if (!(half[i] > 0.0f) || !(half[i] < 1e18f) || !(std::fabs(center[i]) < 1e18f)) return cudaSuccess;
         scale = std::max(scale, std::fabs(center[i]) + half[i]);
     }
+    if (n_tri <= 0) return cudaSuccess;
     size_t free_b = 0, total_b = 0;
-    if (n_tri <= 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    const uint64_t budget = std::min<uint64_t>(free_b / 8, kMaxRecordBytes);
+    cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+    if (e != cudaSuccess) return e;
+    const uint64_t budget = std::min<uint64_t>(free_b / 8, kMaxBytes);
     // Rounding: positions, the records and the transport's own test are single
     // precision at magnitudes up to `scale` (half an ulp: 6e-8 scale); 4e-6
     // leaves a factor of sixty.  0.02 nm on top keeps steps that graze a
@@ -528,12 +529,15 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         g.ny = int(dims[1]);
         g.nz = int(dims[2]);
         const uint64_t cells = uint64_t(g.nx) * g.ny * g.nz;
+        if (cells * sizeof(int32_t) > budget) continue;
         // counting pass: the first words and the counts start at zero
         Block first;
         const size_t at_totals = first.reserve<unsigned long long>(4), at_n_big = first.reserve<uint32_t>(1),
                      at_count = first.reserve<uint32_t>(cells), zeroed = first.used,
                      at_big = first.reserve<int32_t>(uint64_t(n_tri));
-        if (!first.alloc() || cudaMemsetAsync(first.p, 0, zeroed, s) != cudaSuccess) return false;
+        e = first.alloc();
+        if (e == cudaErrorMemoryAllocation) continue;
+        if (e != cudaSuccess || (e = cudaMemsetAsync(first.p, 0, zeroed, s)) != cudaSuccess) return e;
         unsigned long long* const totals = first.at<unsigned long long>(at_totals);
         uint32_t *const n_big = first.at<uint32_t>(at_n_big), *const count = first.at<uint32_t>(at_count);
         int32_t* const big = first.at<int32_t>(at_big);
@@ -543,22 +547,25 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         big_kernel<false><<<blocks, 256, 0, s>>>(tri, g, l, big, n_big);
         total_kernel<<<blocks, 256, 0, s>>>(count, cells, totals);
         unsigned long long used[2] = {0, 0};
-        if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpyAsync(used, totals, 16, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-            return false;
-        if (used[0] * kBrickCells * kRecordBytes > budget || used[1] * 4 > budget) continue;
+        if ((e = cudaGetLastError()) != cudaSuccess ||
+            (e = cudaMemcpyAsync(used, totals, 16, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(s)) != cudaSuccess)
+            return e;
         Block lists, map;
         const size_t at_entry = lists.reserve<int32_t>(used[1]), at_start = lists.reserve<uint64_t>(used[0]),
                      at_cell = lists.reserve<uint32_t>(used[0]), at_cursor = lists.reserve<uint32_t>(used[0]);
         const size_t at_rec = map.reserve<float4>(std::max<uint64_t>(used[0], 1) * kBrickCells * 2),
                      at_top = map.reserve<int32_t>(cells);
-        if (!lists.alloc() || !map.alloc()) return false;
+        if (map.used > budget || lists.used > budget) continue;
+        e = lists.alloc();
+        if (e == cudaSuccess) e = map.alloc();
+        if (e == cudaErrorMemoryAllocation) continue;
+        if (e != cudaSuccess) return e;
         uint32_t *const brick_cell = lists.at<uint32_t>(at_cell), *const cursor = lists.at<uint32_t>(at_cursor);
         uint64_t* const start = lists.at<uint64_t>(at_start);
         int32_t* const top = map.at<int32_t>(at_top);
         float4* const rec = map.at<float4>(at_rec);
-        if (cudaMemsetAsync(cursor, 0, 4 * std::max<uint64_t>(used[0], 1), s) != cudaSuccess) return false;
+        if ((e = cudaMemsetAsync(cursor, 0, 4 * std::max<uint64_t>(used[0], 1), s)) != cudaSuccess) return e;
         assign_kernel<<<blocks, 256, 0, s>>>(count, g, totals + 2, top, start, brick_cell);
         l.top = top;
         l.start = start;
@@ -569,8 +576,9 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         if (used[0])
             record_kernel<<<unsigned(used[0]), unsigned(kBrickCells), 0, s>>>(tri, g, brick_cell, start, cursor, l.entry,
                                                                               margin, rounding, rec);
-        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return false;
+        if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
         out->memory = map.p;
+        out->bytes = map.used;
         map.p = nullptr;
         dev::Clearance& m = out->map;
         m.top = top;
@@ -587,9 +595,9 @@ bool build_clearance(const float4* tri, int n_tri, const float center[3], const 
         m.ny = g.ny;
         m.reach = reach;
         m.far_reach = g.cell;
-        return true;
+        return cudaSuccess;
     }
-    return false;
+    return cudaSuccess;
 }
 
 void free_clearance(ClearanceMap* m) {

@@ -12,13 +12,14 @@ namespace nbx {
 struct ClearanceMap {
     dev::Clearance map{};   // what the kernels take; map.top == nullptr: no map
     void* memory = nullptr;   // the device allocation behind it
+    size_t bytes = 0;         // its size
 };
 
 // Builds the map of `n_tri` triangles (three float4 each, device memory) over
-// the octree's root box.  False (and nothing allocated) when the memory for it
-// is not there or a launch failed: the transport then walks every step.
-bool build_clearance(const float4* tri, int n_tri, const float center[3], const float half[3], int sms, cudaStream_t s,
-                     ClearanceMap* out);
+// the octree's root box.  Without memory for it the call succeeds with an empty
+// map (the transport then walks every step); every other error is returned.
+cudaError_t build_clearance(const float4* tri, int n_tri, const float center[3], const float half[3], int sms,
+                            cudaStream_t s, ClearanceMap* out);
 void free_clearance(ClearanceMap* m);
 
 }  // namespace nbx

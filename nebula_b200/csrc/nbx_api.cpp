@@ -629,13 +629,11 @@ int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* o) {
         g.tri = ctx->tris.p;
         g.tri_face = ctx->tri_faces.p;
         g.tri_plane = ctx->tri_planes.p;
-        // without memory for the map the transport walks every step
         nbx::free_clearance(&ctx->clearance);
-        if (nbx::build_clearance(ctx->tris.p, int(o->n_triangles), o->center, o->halfsize, ctx->sms, ctx->stream,
-                                 &ctx->clearance))
-            g.clear = ctx->clearance.map;
-        else
-            g.clear = nbx::dev::Clearance{};
+        g.clear = nbx::dev::Clearance{};
+        ck(nbx::build_clearance(ctx->tris.p, int(o->n_triangles), o->center, o->halfsize, ctx->sms, ctx->stream,
+                                &ctx->clearance), "clearance map");
+        g.clear = ctx->clearance.map;
         g.cx = o->center[0];
         g.cy = o->center[1];
         g.cz = o->center[2];
@@ -654,6 +652,14 @@ int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* o) {
         ctx->have_geometry = true;
         return NBX_OK;
     });
+}
+
+int nbx_get_clearance(nbx_ctx* ctx, float* cell, uint64_t* bytes) {
+    if (!ctx || !cell || !bytes) return NBX_ERR_ARG;
+    if (!ctx->have_geometry) return fail(ctx, NBX_ERR_STATE, "nbx_get_clearance before nbx_set_geometry");
+    *cell = ctx->clearance.map.h;
+    *bytes = ctx->clearance.bytes;
+    return NBX_OK;
 }
 
 int nbx_add_material(nbx_ctx* ctx, const nbx_material* m) {

@@ -193,6 +193,47 @@ def test_fine_mesh_in_a_vast_domain():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("spare", [1500, 400])
+def test_map_when_memory_is_short(spare, inputs):
+    """With little device memory left the map takes an eighth of it at most,
+    its coarse grid included (here 200 MB at the usual cell), and larger cells
+    before it is given up; runs are the same."""
+    import nebula_b200 as nb
+    import torch
+    from nebula_b200 import generators as g
+    far = np.zeros(1, formats.TRI_DTYPE)   # one small triangle that makes the domain 6 um wide
+    far["v"] = np.array([5700.0, 5700.0, -5700.0]) + np.array([[0, 0, 0], [5, 0, 0], [0, 5, 0]])
+    far["mat_in"] = far["mat_out"] = formats.VACUUM
+    tris = np.concatenate([g.cube_geometry(size=(300.0, 300.0, 300.0)), far])
+    recs = g.scan_beam(8, 8, 8, 500.0, z_start=1.0, seed=2)
+    o = nb.HostOctree(nb.triangles_from_tri_array(tris))
+    got = []
+    for short in (True, False):
+        ctx = nb.Context(device=0, seed=3)
+        ctx.add_material(nb.HostMaterial(inputs["si"]))
+        hold = None
+        if short:
+            torch.cuda.init()
+            hold = torch.empty(torch.cuda.mem_get_info()[0] - (spare << 20), dtype=torch.uint8, device="cuda")
+        free = torch.cuda.mem_get_info()[0]
+        ctx.set_geometry(o)
+        took = free - torch.cuda.mem_get_info()[0]
+        if short:
+            assert took < free // 8 + (16 << 20), (took, free)   # (and a few MB of triangles, in 2 MB pages)
+        m = ctx.clearance()
+        assert 0 < m["bytes"] <= took
+        assert m["cell"] > 4 if short else m["cell"] == 4
+        ctx.set_tag_range(len(recs))
+        ctx.push_records(recs)
+        ctx.run()
+        got.append(np.stack(ctx.tag_counts(0, len(recs))))
+        ctx.close()
+        del hold
+        torch.cuda.empty_cache()
+    assert np.array_equal(*got) and got[0].sum() > 0
+
+
+@pytest.mark.gpu
 def test_table_indices_at_the_edges(inputs):
     """Table lookups whose index is clamped: below and above the axes, on
     every grid point and its neighbours, huge, infinite and NaN coordinates
