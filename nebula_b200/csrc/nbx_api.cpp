@@ -601,8 +601,6 @@ const char* nbx_last_error(nbx_ctx* ctx) { return ctx ? ctx->err.c_str() : g_thr
 int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* o) {
     if (!ctx || !o || !o->octree_data || o->n_octree < 8 || !o->triangles) return NBX_ERR_ARG;
     return guarded(ctx, [&] {
-        ctx->octree.alloc(o->n_octree);
-        to_device(ctx, ctx->octree.p, o->octree_data, sizeof(int32_t) * o->n_octree, "octree");
         std::vector<float4> t(3 * std::max<uint64_t>(o->n_triangles, 1));
         for (uint64_t i = 0; i < o->n_triangles; ++i) {
             const nbx_triangle& s = o->triangles[i];
@@ -615,6 +613,11 @@ int nbx_set_geometry(nbx_ctx* ctx, const nbx_octree* o) {
             t[3 * i + 1] = make_float4(s.e1[0], s.e1[1], s.e1[2], b);
             t[3 * i + 2] = make_float4(s.e2[0], s.e2[1], s.e2[2], 0.0f);
         }
+        // From here on the old geometry is gone: a failure (no memory) leaves none,
+        // not the new octree with the old triangles.
+        ctx->have_geometry = false;
+        ctx->octree.alloc(o->n_octree);
+        to_device(ctx, ctx->octree.p, o->octree_data, sizeof(int32_t) * o->n_octree, "octree");
         ctx->tris.alloc(t.size());
         to_device(ctx, ctx->tris.p, t.data(), sizeof(float4) * t.size(), "triangles");
         ctx->tri_faces.alloc(std::max<uint64_t>(o->n_triangles, 1));

@@ -193,6 +193,47 @@ def test_fine_mesh_in_a_vast_domain():
 
 
 @pytest.mark.gpu
+def test_refused_geometry_changes_nothing(inputs):
+    """A geometry that nbx_set_geometry refuses leaves the one before it whole;
+    one that fails for want of memory leaves none."""
+    import nebula_b200 as nb
+    import torch
+    from nebula_b200 import generators as g
+    ctx = nb.setup(inputs["cube"], [inputs["si"]], device=0, seed=3)
+    recs = g.scan_beam(8, 8, 8, 500.0, z_start=1.0, seed=2)
+    ctx.set_tag_range(len(recs))
+    other = nb.HostOctree(nb.triangles_from_tri_array(inputs["rough"]))
+    other._p.contents.triangles[5].mat_in = 40000
+    got = []
+    for again in (False, True):
+        if again:
+            with pytest.raises(nb.NbxError) as e:
+                ctx.set_geometry(other)
+            assert e.value.code == -1
+        ctx.reset_tallies()
+        ctx.set_uid_base(0)
+        ctx.push_records(recs)
+        ctx.run()
+        got.append(np.stack(ctx.tag_counts(0, len(recs))))
+    assert np.array_equal(*got) and got[0].sum() > 0
+    other._p.contents.triangles[5].mat_in = 0
+    big = nb.HostOctree(nb.triangles_from_tri_array(g.rough_geometry(n=256, size=500.0)))
+    hold = [torch.empty(torch.cuda.mem_get_info()[0] - (4 << 20), dtype=torch.uint8, device="cuda")]
+    with pytest.raises(nb.NbxError) as e:
+        ctx.set_geometry(big)
+    assert e.value.code == -2
+    hold.clear()
+    torch.cuda.empty_cache()
+    with pytest.raises(nb.NbxError) as e:
+        ctx.run()
+    assert e.value.code == -6
+    ctx.set_geometry(big)
+    ctx.push_records(recs)
+    ctx.run()
+    ctx.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("spare", [1500, 400])
 def test_map_when_memory_is_short(spare, inputs):
     """With little device memory left the map takes an eighth of it at most,
