@@ -341,3 +341,46 @@ def test_launch_shapes_and_shallow_stacks_change_nothing(mode, inputs):
         for a, b in zip(got, want):
             assert all(np.array_equal(x, y) for x, y in zip(a, b)), (variant, block, depth)
     assert want[0][0].sum() > 100 and want[2][-1] == 0
+
+
+@pytest.mark.gpu
+def test_sample_mode_covers_the_queue(inputs):
+    """Sample mode takes every primary once, whatever its launch shape and the
+    ranges the queue is cut into (one, several an SM, fewer primaries than
+    ranges, one shared cursor): the event totals of a plain run, and the same
+    set of samples each time."""
+    import nebula_b200 as nb
+    from nebula_b200 import generators as g
+    recs = g.scan_beam(60, 40, 16, 500.0, spacing=2.0, origin=(-60.0, -40.0), seed=9)   # 38,400: two ranges an SM
+    keys = ("primaries_done", "steps", "events_elastic", "events_inelastic", "events_boundary", "secondaries",
+            "terminated", "detected_se", "detected_bse")
+    want = None
+    for mode, shape, shared in (("plain", (3, 256), 0), ("sample", (3, 256), 0), ("sample", (2, 32), 0),
+                                ("sample", (7, 128), 0), ("sample", (4, 256), 1)):
+        ctx = nb.setup(inputs["grating_small"], [inputs["si"]], device=0, seed=5, shared_pop=shared)
+        ctx.set_tag_range(len(recs))
+        ctx.build_surface_map([-150, -150, -60], [150, 150, 60], 2.0, 20.0)
+        ctx.set_tuning(*shape, 64, 2)
+        if mode == "sample":
+            ctx.set_sample_capacity(1 << 21)
+            ctx.set_mode("sample")
+        got = []
+        for n in (len(recs), 149, 1):
+            ctx.reset_tallies()
+            ctx.set_uid_base(0)
+            ctx.push_records(recs[:n])
+            ctx.run()
+            s = ctx.stats()
+            got.append([s[k] for k in keys])
+            assert s["primaries_done"] == n
+            if mode == "sample":
+                x = np.column_stack(ctx.get_samples(1 << 21, with_cost=True))
+                got.append(x[np.lexsort(x.T)])
+        ctx.close()
+        if mode == "plain":
+            totals = got
+            continue
+        assert got[0::2] == totals, (shape, shared)
+        want = want or got[1::2]
+        assert all(np.array_equal(a, b) for a, b in zip(got[1::2], want)), (shape, shared)
+    assert len(want[0]) > 1000
