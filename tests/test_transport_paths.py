@@ -308,10 +308,8 @@ def test_table_indices_at_the_edges(inputs):
 @pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["plain", "weighted", "network"])
 def test_launch_shapes_and_shallow_stacks_change_nothing(mode, inputs):
-    """The same per-primary tallies whatever the launch shape, with stacks of
-    one electron per thread (secondaries then go through the next generations'
-    queues, in learned mode with their weights) and with queues that fill whole
-    ranges, one primary and none."""
+    """The same per-primary tallies whatever the launch shape and the stacks'
+    depth, and with queues that fill whole ranges, one primary and none."""
     import nebula_b200 as nb
     from nebula_b200 import generators as g
     recs = g.scan_beam(16, 12, 11, 2000.0, spacing=4.0, origin=(-32.0, -24.0), seed=9)
@@ -341,6 +339,64 @@ def test_launch_shapes_and_shallow_stacks_change_nothing(mode, inputs):
         for a, b in zip(got, want):
             assert all(np.array_equal(x, y) for x, y in zip(a, b)), (variant, block, depth)
     assert want[0][0].sum() > 100 and want[2][-1] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["plain", "weighted", "network"])
+def test_secondaries_through_the_queue(mode, inputs):
+    """Stacks of one electron per thread and enough primaries for a warp to
+    fill its 32: secondaries then go through the next generations' queues (in
+    learned mode with their weights), and every tally is that of a run that needs
+    no queue."""
+    import nebula_b200 as nb
+    from nebula_b200 import generators as g
+    recs = g.scan_beam(40, 40, 25, 5000.0, spacing=2.0, origin=(-40.0, -40.0), seed=9)
+    got = []
+    for shape in ((3, 256, 64), (2, 32, 1)):
+        ctx = nb.setup(inputs["grating_small"], [inputs["si"]], device=0, seed=5, capacity=1 << 24)
+        ctx.set_tag_range(len(recs))
+        if mode != "plain":
+            ctx.build_surface_map([-150, -150, -60], [150, 150, 60], 2.0, 20.0)
+            ctx.mlp_set_params(nb.mlp_init_params(3))
+            ctx.set_mode("learned", rr_threshold=0.3, split_threshold=0.3, max_roulette_exp=3)
+            if mode == "weighted":
+                ctx.set_importance_table(16, 16, 8)
+        ctx.set_tuning(*shape, 2)
+        ctx.push_records(recs)
+        ctx.run()
+        s = ctx.stats()
+        assert (s["generations"] > 1) == (shape[2] == 1), s["generations"]
+        got.append(list(ctx.tag_counts(0, len(recs))) + list(ctx.tag_weights(0, len(recs))) +
+                   [s[k] for k in ("steps", "events_elastic", "events_inelastic", "events_boundary", "secondaries",
+                                   "splits", "roulette_killed", "terminated", "detected", "primaries_done")])
+        assert s["queue_overflow"] == 0 and s["primaries_done"] == len(recs)
+        if mode != "plain":
+            assert got[-1][2].sum() < 0.75 * got[-1][0].sum()   # most secondaries carry a weight of one half
+        ctx.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.gpu
+def test_deposits_do_not_depend_on_the_launch(inputs):
+    """The same set of energy-deposit records whatever the launch shape."""
+    import nebula_b200 as nb
+    from nebula_b200 import generators as g
+    recs = g.scan_beam(12, 12, 8, 500.0, spacing=4.0, origin=(-24.0, -24.0), seed=9)
+    want = None
+    for shape in ((3, 256, 16), (2, 32, 1), (7, 128, 2), (4, 256, 64)):
+        ctx = nb.setup(inputs["grating_small"], [inputs["si"]], device=0, seed=5, record_deposits=True,
+                       deposit_capacity=1 << 23)
+        ctx.set_tuning(*shape, 2)
+        ctx.push_records(recs)
+        ctx.run()
+        s = ctx.stats()
+        d = ctx.flush_deposits()
+        ctx.close()
+        assert s["deposits_dropped"] == 0 and len(d) == s["deposits"] > 100000
+        x = d.view(np.uint32).reshape(len(d), -1)
+        x = x[np.lexsort(x.T)]
+        want = x if want is None else want
+        assert np.array_equal(x, want), shape
 
 
 @pytest.mark.gpu
