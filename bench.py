@@ -803,7 +803,9 @@ def main():
             "roofline": {"bound": "issue/L1-L2 latency", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "dram_frac": dram_frac, "ncu": ncu,
                          "peak_kind": peak_kind, "bytes_per_event": round(b_event, 2), "bytes_breakdown": b_parts,
-                         "kernel": "transport_kernel"},
+                         "kernel": "transport_kernel",
+                         "note": "counts a walk at every step; the clearance map makes most of them unnecessary, "
+                                 "see dram_frac for the bytes moved"},
             "clocks": clocks,
             "cpu_baseline": cpu,
             "reference_gpu_program": ref_gpu,

@@ -166,11 +166,12 @@ __device__ __forceinline__ float table_importance(const TransportArgs& a, const 
 // bookkeeping.  Now
 //
 // * a step whose free path the clearance map answers goes straight on to its
-//   scattering event; one that needs the walk (about one in eight) goes to the
-//   warp's ring in shared memory and its lane takes other work.  When
-//   kWalkBatch of them wait, or too few lanes have other work, the warp walks
-//   them together, one electron per lane; those that met a triangle cross (or
-//   leave) there, the others come back for their scattering event.
+//   scattering event; one that needs the walk (one in nine on the grating, one
+//   in five on the contact holes) goes to the warp's ring in shared memory and
+//   its lane takes other work.  When kWalkBatch of them wait, or too few lanes
+//   have other work, the warp walks them together, one electron per lane; those
+//   that met a triangle cross (or leave) there, the others come back for their
+//   scattering event.
 // * parked electrons (the parents of running secondaries) lie on one stack per
 //   warp, its top kTop entries in shared memory, the rest in the warp's part
 //   of stack_mem, so any lane that falls idle takes the next one: a cascade
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(MinBlocks == 7 ? 128 : 256, MinBlocks) transpo
     // top_n entries of the stack in shared memory, deep_n below them.
     int head = 0, n_back = 0, n_wait = 0, top_n = 0, deep_n = 0;
     bool have = false, drained = false;
-    // Primaries: this SM's range of the queue first, then the following ones
+    // Primaries: this SM's ranges of the queue first, then the next SMs'
     // (`probe` ranges found used up).
     uint32_t probe = 0, taken = 0;
     uint32_t range = a.range_cursor ? range_at(a, 0) : 0u;

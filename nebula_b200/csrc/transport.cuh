@@ -313,10 +313,10 @@ struct LeafCache {
 // distance in (0, reach], judged from the triangle's plane alone: the plane
 // is behind the ray, or farther along it than `reach`, by more than the
 // rounding of both this test and the exact one (the unit of the scaled plane
-// record, see triangle_faces_kernel).  Never true for a triangle that intersect_ray would accept at such a distance; not true
-// for non-finite input.  Ten multiply-adds and one 16-byte gather in place of
-// the face test and Moeller-Trumbore, which about half of a leaf's triangles
-// used to reach.
+// record, see triangle_faces_kernel).  Never true for a triangle that
+// intersect_ray would accept at such a distance; not true for non-finite input.
+// Six multiply-adds and one 16-byte gather in place of the face test and
+// Moeller-Trumbore, which about half of a leaf's triangles used to reach.
 __device__ __forceinline__ bool plane_misses(const Geometry& g, int ti, V3 start, V3 dir, float reach) {
     const float4 p = __ldg(g.tri_plane + ti);
     const float h = p.w - __fmaf_rn(p.x, start.x, __fmaf_rn(p.y, start.y, p.z * start.z));
