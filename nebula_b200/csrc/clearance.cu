@@ -19,19 +19,26 @@
 // margin, on flat faces); the second one serves edges and corners.
 //
 // The margin covers the rounding of the exact test, because "meets no
-// triangle" has to mean that intersect_ray reports no hit.  With u = 2^-24,
-// |s| the distance from the triangle's corner to the ray's start and k =
-// |e1||e2| / |e1 x e2|, the test's three numerators are off by at most
-// 12 u |s| times the edges in them and its determinant by 8 u |e1||e2|, so the
-// point that it reports lies within 44 u k |s| / cos of the triangle, cos being
-// that of the ray's angle to the triangle's normal, and along that normal
-// within 12 u k |s|.  A triangle's `slack` is 24 u k |s| plus the 2.4e-6 of its
-// edges by which the test enlarges it; at an angle phi to its slab it widens
-// the slab by slack / 2 + 10 slack sin(phi), which covers rays down to a cosine
-// of 0.18 at the bound and of 0.02 at the errors that occur (a tenth of it),
-// and it is a candidate of the cells within 10 slack.  Triangles of sound
-// meshes mostly have a slack below 0.01 nm, and the margin decides; strips of
-// 1000 nm x 0.3 nm (5 nm) make the cells round them walk.  With one margin for
+// triangle" has to mean that intersect_ray reports no hit.  With u = 2^-24, s
+// the vector from the triangle's corner to the ray's start and k = |e1||e2| /
+// |e1 x e2|, the test's numerators u and v are off by at most 12 u |s| times the
+// edge in them, its determinant by 8 u |e1||e2| and the numerator of t by
+// 6 u |e2| . (|s| x |e1|), the triple product of the vectors' magnitudes by
+// component with its differences taken as sums.  So the point that it reports
+// lies
+// * along the triangle's normal within that triple product's 6 u / |e1 x e2|
+//   (small where the plane runs along an axis, 12 u k |s| at most) and 8 u k
+//   times the step,
+// * in the triangle's plane within 44 u k |s| / cos of it, cos being that of the
+//   ray's angle to the normal, and the 2.4e-6 of the edges by which the test
+//   enlarges a triangle.
+// A triangle at an angle phi to its slab widens the slab by the first and by the
+// second times sin(phi), with 240 u in place of 44 u / cos: rays down to a cosine
+// of 0.18 at the bound and of 0.02 at the errors that occur (a tenth of it).  It
+// is a candidate of the cells that its plane meets within the first bound and
+// that lie within the second of it.  On the benchmark scans all this is below
+// 0.01 nm for most triangles, and the margin decides; strips of 1000 nm x 0.3 nm
+// at an angle to one another make the cells round them walk.  With one margin for
 // all shapes, runs through sheets of strips had 4 of 35,305 crossings fewer
 // than the walk reports (4000 nm x 4 nm) and 247 of 28,966 (8000 nm x 1 nm).
 //
@@ -65,12 +72,18 @@ struct Grid {
 struct alignas(16) TriBox {
     float3 a, e1, e2, lo, hi;
     float3 u;      // unit normal (zero without an area)
-    float slack;   // rounding of the exact test (nm; infinite without an area)
-    float grow;    // boxes within this distance (nm) count as near
+    float k;       // |e1||e2| / |e1 x e2| (infinite without an area)
+    float inv;     // 1 / |e1 x e2|
+    float size;    // diagonal of the bounding box
+    float thick;   // rounding of the exact test along the normal, at most (nm)
+    float grow;    // and in the plane (nm)
 };
 
 __device__ __forceinline__ float min3(float a, float b, float c) { return fminf(a, fminf(b, c)); }
 __device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(a, fmaxf(b, c)); }
+
+constexpr float kUnit = 5.9604645e-8f;         // 2^-24
+constexpr float kReachDiagonal = 1.7320508f;   // of a cube of edge 1
 
 // The normal is formed in double precision: that of a needle would be lost in
 // single precision, and with it the plane test of near_box.
@@ -88,26 +101,28 @@ __device__ __forceinline__ TriBox load_tri(const float4* tri, int t, const Grid&
     const double s = l2 > 0.0 ? rsqrt(l2) : 0.0;
     r.u = make_float3(float(nx * s), float(ny * s), float(nz * s));
     const float b2 = B.x * B.x + B.y * B.y + B.z * B.z, c2 = C.x * C.x + C.y * C.y + C.z * C.z;
-    const float k = s > 0.0 ? sqrtf(b2) * sqrtf(c2) * float(s) : INFINITY;
+    r.k = s > 0.0 ? sqrtf(b2) * sqrtf(c2) * float(s) : INFINITY;
+    r.inv = s > 0.0 ? float(s) : INFINITY;
     const float dx = r.hi.x - r.lo.x, dy = r.hi.y - r.lo.y, dz = r.hi.z - r.lo.z;
-    const float size = sqrtf(dx * dx + dy * dy + dz * dz);   // at least the longest edge
-    const float near = 1.75f * (g.cell / kBrick + 2.0f * g.reach);   // diagonal of a widened fine cell
-    r.slack = 24.0f * 5.9604645e-8f * k * (size + near) + 2.4e-6f * size;
-    r.grow = fminf(10.0f * r.slack, fminf(2.0f * size, 8.0f * g.cell));
+    r.size = sqrtf(dx * dx + dy * dy + dz * dz);   // at least the longest edge
+    // |s| of rays in a widened fine cell near the triangle (kReachDiagonal: its diagonal)
+    const float far = 1.25f * r.size + kReachDiagonal * (g.cell / kBrick + 2.0f * g.reach);
+    r.thick = 20.0f * kUnit * r.k * far;
+    r.grow = fminf(240.0f * kUnit * r.k * far + 2.4e-6f * r.size, fminf(2.0f * r.size, 8.0f * g.cell));
     return r;
 }
 
 // Conservative triangle / box test: bounding boxes, then the triangle's
 // plane against the box.  (cx, cy, cz) is the box centre, h its half edge.
 __device__ __forceinline__ bool near_box(const TriBox& t, float cx, float cy, float cz, float h) {
-    h += t.grow;
-    if (t.lo.x > cx + h || t.hi.x < cx - h || t.lo.y > cy + h || t.hi.y < cy - h || t.lo.z > cz + h || t.hi.z < cz - h)
+    const float w = h + t.grow;
+    if (t.lo.x > cx + w || t.hi.x < cx - w || t.lo.y > cy + w || t.hi.y < cy - w || t.lo.z > cz + w || t.hi.z < cz - w)
         return false;
     const float x = t.a.x - cx, y = t.a.y - cy, z = t.a.z - cz;
     const float d = t.u.x * x + t.u.y * y + t.u.z * z;
     // 1e-6, 1.0001: rounding of the normal, the difference and the two sums
     const float r = (fabsf(t.u.x) + fabsf(t.u.y) + fabsf(t.u.z)) * h * 1.0001f + 1e-6f * (fabsf(x) + fabsf(y) + fabsf(z));
-    return !(fabsf(d) > r);
+    return !(fabsf(d) > r + t.thick);
 }
 
 __device__ __forceinline__ int clamp_cell(float x, int n) {
@@ -350,7 +365,16 @@ struct Slab {
                                            float rounding) {
         const float3 p = make_float3(b.a.x - px, b.a.y - py, b.a.z - pz);
         const float co = b.u.x * u.x + b.u.y * u.y + b.u.z * u.z;
-        const float m = fmaxf(margin, b.slack * (0.5f + 10.0f * sqrtf(fmaxf(1.0f - co * co, 0.0f)))) + rounding;
+        // magnitudes of s by component and in length, for rays that start in the box
+        const float sx = fabsf(p.x) + box, sy = fabsf(p.y) + box, sz = fabsf(p.z) + box;
+        const float ex = fabsf(b.e1.x), ey = fabsf(b.e1.y), ez = fabsf(b.e1.z);
+        const float triple = fabsf(b.e2.x) * (sy * ez + sz * ey) + fabsf(b.e2.y) * (sz * ex + sx * ez) +
+                             fabsf(b.e2.z) * (sx * ey + sy * ex);
+        const float along = kUnit * (6.0f * triple * b.inv + 8.0f * b.k * kReachDiagonal * box);
+        const float across = 240.0f * kUnit * b.k * sqrtf(sx * sx + sy * sy + sz * sz) + 2.4e-6f * b.size;
+        // (k is infinite without an area: no bound)
+        const float si = sqrtf(fmaxf(1.0f - co * co, 0.0f)) + 5e-4f;   // (rounding of co near 1)
+        const float m = b.k < 1e30f ? fmaxf(margin, along + across * si) + rounding : INFINITY;
         float x, y;
         if (clipped_extent(b, p, box + b.grow, u, 0.1f * margin, x, y)) {
             lo = fminf(lo, x - m);
@@ -378,9 +402,9 @@ struct Slab {
 // times (nearest; normal, and the second slab's nearest; extent, and the second
 // slab's normal; the second slab's extent).  B200, against every thread reading
 // and preparing every candidate six times and clipping polygons in local
-// memory: 16 x 16 contact holes (89,079 bricks, 2.8 million candidates) 16.2 ->
-// 5.6 ms, 8 x 8 holes 4.5 -> 1.6 ms; nbx_set_geometry 29.2 -> 19.5 and 9.0 ->
-// 7.8 ms, of which 11 and 3 ms are the octree and the triangles.
+// memory: 16 x 16 contact holes (89,067 bricks, 2.8 million candidates) 16.2 ->
+// 6.7 ms, 8 x 8 holes 4.5 -> 1.8 ms; nbx_set_geometry 29 -> 21 and 9.0 -> 6.9 ms,
+// of which 11 and 3 ms are the octree and the triangles.
 //
 // A brick of more than kMaxList candidates (a mesh far finer than the cells, as
 // in a domain that is far larger) gets records under which every step walks:
