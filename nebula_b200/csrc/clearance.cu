@@ -109,6 +109,11 @@ __device__ __forceinline__ TriBox load_tri(const float4* tri, int t, const Grid&
     const float far = 1.25f * r.size + kReachDiagonal * (g.cell / kBrick + 2.0f * g.reach);
     r.thick = 20.0f * kUnit * r.k * far;
     r.grow = fminf(240.0f * kUnit * r.k * far + 2.4e-6f * r.size, fminf(2.0f * r.size, 8.0f * g.cell));
+    // The exact test drops a triangle whose determinant is below kEps, rounding
+    // included, for every ray: it is near nothing (exported meshes hold many
+    // such triangles, of no area and short edges, on their surfaces).
+    if (l2 < 1e-10 && sqrtf(float(l2)) + 10.0f * kUnit * sqrtf(b2) * sqrtf(c2) < 0.99f * dev::kEps)
+        r.lo = make_float3(INFINITY, INFINITY, INFINITY);
     return r;
 }
 
@@ -397,10 +402,10 @@ struct Slab {
 // candidates' clipped parts, each widened by its margin.
 //
 // Bound by the instructions of clipped_extent and near_box (a brick of the
-// contact holes has 31 candidates, each near a third of its cells).  The block
-// keeps its candidates in shared memory, 64 at a time, and goes over them four
-// times (nearest; normal, and the second slab's nearest; extent, and the second
-// slab's normal; the second slab's extent).  B200, against every thread reading
+// contact holes has 31 candidates).  The block keeps its candidates in shared
+// memory, 64 at a time, and goes over them four times (nearest; normal, and the
+// second slab's nearest; extent, and the second slab's normal; the second slab's
+// extent).  B200, against every thread reading
 // and preparing every candidate six times and clipping polygons in local
 // memory: 16 x 16 contact holes (89,067 bricks, 2.8 million candidates) 16.2 ->
 // 6.7 ms, 8 x 8 holes 4.5 -> 1.8 ms; nbx_set_geometry 29 -> 21 and 9.0 -> 6.9 ms,

@@ -174,7 +174,7 @@ struct nbx_ctx {
     double last_run_ms = 0, last_kernel_ms = 0;
     int block = 256, bpsm = 0, variant = 3;
     int stack_depth = 16;   // parked electrons per thread before a secondary goes to the next generation
-    int chunk = 8;          // generation launches queued between two 4-byte host reads
+    int chunk = 8;          // generation launches queued between two host reads
     uint64_t queue_capacity = 0;   // overflow-queue entries of the last run
     // device address of the allocation-free transport's scratch array,
     // looked up by this context's first nbx_run_noalloc call
@@ -886,8 +886,8 @@ int nbx_run(nbx_ctx* ctx) {
         ctx->generations = 0;
         ctx->last_run_ms = ctx->last_kernel_ms = 0;
         if (ctx->n_queued == 0) return NBX_OK;
-        // Overflow-queue capacity (secondaries of cascades deeper than the
-        // per-thread stack): explicit, else one per queued primary (at least
+        // Overflow-queue capacity (secondaries born with their warp's stack
+        // full): explicit, else one per queued primary (at least
         // 1M), bounded by a quarter of the free device memory.
         uint64_t want = ctx->cfg.capacity ? ctx->cfg.capacity : std::max<uint64_t>(1ull << 20, ctx->n_queued);
         want = std::min<uint64_t>(want, 0xFFFFFFF0ull);
