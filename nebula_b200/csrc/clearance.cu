@@ -108,6 +108,8 @@ __device__ __forceinline__ TriBox load_tri(const float4* tri, int t, const Grid&
     // |s| of rays in a widened fine cell near the triangle (kReachDiagonal: its diagonal)
     const float far = 1.25f * r.size + kReachDiagonal * (g.cell / kBrick + 2.0f * g.reach);
     r.thick = 20.0f * kUnit * r.k * far;
+    // (capped: a hit farther off than twice the triangle's size takes a ray whose
+    // line meets it to one part in 1e7 and a distance that is all rounding)
     r.grow = fminf(240.0f * kUnit * r.k * far + 2.4e-6f * r.size, fminf(2.0f * r.size, 8.0f * g.cell));
     // The exact test drops a triangle whose determinant is below kEps, rounding
     // included, for every ray: it is near nothing (exported meshes hold many
